@@ -28,20 +28,9 @@ __global__ void k_design_record(Geom g, const int4* __restrict__ edges, int n, c
     const long long slot = (long long)step_index(counter) - *base;
     if (slot < 0 || slot >= cap) return;
     const int4 d = edges[t];
-    const int c = d.x;
-    const int p[3] = {d.y, d.z, d.w};
-    const int U = (c + 1) % 3, V = (c + 2) % 3;
-    const long long st[3] = {(long long)g.n1 * g.p2, g.p2, 1};
-    const long long id = ((long long)p[0] * g.n1 + p[1]) * g.p2 + p[2];
-    const float a = h_new[V * g.cs + id] - h_new[V * g.cs + id - st[U]];
-    const float b = h_new[U * g.cs + id] - h_new[U * g.cs + id - st[V]];
-    const AxisNode& au = g.ax[U][p[U]];
-    const AxisNode& av = g.ax[V][p[V]];
-    float t1 = a * au.inv_dd, t2 = b * av.inv_dd;
-    if (au.slot_e >= 0) t1 += psi[g.psi_off[c * 3 + U] + psi_at(g, U, p[0], p[1], p[2], au.slot_e)];
-    if (av.slot_e >= 0) t2 += psi[g.psi_off[c * 3 + V] + psi_at(g, V, p[0], p[1], p[2], av.slot_e)];
-    hist_e[slot * n + t] = e_in[c * g.cs + id];
-    hist_s[slot * n + t] = t1 - t2;
+    const long long id = ((long long)d.y * g.n1 + d.z) * g.p2 + d.w;
+    hist_e[slot * n + t] = e_in[d.x * g.cs + id];
+    hist_s[slot * n + t] = design_curl(g, d, h_new, psi);
 }
 
 // Each E edge's (ca, cb) where its update runs (cb != 0, off the low faces), else (1, 0): the

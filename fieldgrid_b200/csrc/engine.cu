@@ -24,6 +24,7 @@
 #include "stencil_shell.cuh"
 #include "stencil_tma.cuh"
 #include "stencil_tb2.cuh"
+#include "stencil_resident.cuh"
 #include "setup_kernels.cuh"
 #include "adjoint_kernels.cuh"
 
@@ -124,6 +125,16 @@ int staged_upload(Gpu* g, void* dst, const void* src, size_t bytes, void* stream
     const char* s8 = static_cast<const char*>(src);
     return staged_fill(g, dst, bytes, st, [s8](char* buf, size_t off, size_t n) { std::memcpy(buf, s8 + off, n); });
 }
+
+// Steps of one resident launch at most (a bound on the time one kernel holds the GPU).
+constexpr uint64_t RES_MAX_STEPS = 1024;
+// Nodes of a grid stepped resident at most: beyond, the fields and psi (24 to 35 B per node) leave the
+// L2. Measured per step against the TMA march's graphs and the separate kernels': 65^3 10.0 us against
+// 35.1 and 21.1; 121^3 with Debye spheres 31 against 64 and 57; 160^3 85 against 110 and 161.
+constexpr long long RES_MAX_NODES = 4 << 20;
+// 4-node groups of a grid stepped by one cluster at most: its barrier is shorter than a grid-wide one,
+// but 16 SMs share the work (29x19x14: 4.1 us a step against 5.2; 25^3: 6.5 against 6.5).
+constexpr long long RES_CLUSTER_GROUPS = 4096;
 
 struct Session {
     Gpu* gpu = nullptr;
@@ -267,6 +278,13 @@ struct Session {
     cudaEvent_t shell_fork = nullptr, shell_join = nullptr;
     int prio_lo = 0, prio_hi = 0;
     bool capturing = false;
+    // whole calls of session_step as one resident launch (stencil_resident.cuh), where the grid's
+    // state stays in L2
+    bool resident = false;
+    int res_blocks = 0, res_groups = 0;
+    bool res_cluster = false;
+    bool k_quads = false;           // a grid of that size, its k slots numbered by 4-node groups
+    unsigned* res_bar = nullptr;    // the grid barrier's arrivals
     std::map<int, cudaGraphExec_t> slot_graphs;      // captured steps by (kind, phase t mod 6)
     std::vector<void*> extra_allocs;
 };
@@ -704,6 +722,129 @@ int enqueue_step(Session& s, int parity, std::string& err) {
     }
     mark(nullptr);
     return FG_OK;
+}
+
+// ---- resident stepping ----------------------------------------------------------------------
+
+template <typename F>
+int with_resident(int cid_bytes, bool cluster, F&& f) {
+    if (cid_bytes == 1) return cluster ? f(k_resident<uint8_t, true>) : f(k_resident<uint8_t, false>);
+    if (cid_bytes == 2) return cluster ? f(k_resident<uint16_t, true>) : f(k_resident<uint16_t, false>);
+    return cluster ? f(k_resident<uint32_t, true>) : f(k_resident<uint32_t, false>);
+}
+
+// Whether a session's steps run resident, and its launch shape.
+int plan_resident(Session& s, std::string& err) {
+    const Geom& g = s.geom;
+    s.resident = false;
+    if (!s.k_quads) return FG_OK;
+    int coop = 0, sms = 0, per = 0;
+    FG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s.gpu->device));
+    FG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.gpu->device));
+    if (!coop) return FG_OK;
+    const long long total = (long long)g.n0 * g.n1 * ((g.n2 + 3) / 4);
+    auto groups_of = [&](long long blocks) {   // per block and pass, in whole warps
+        return int(std::min<long long>(RES_GROUPS, std::max<long long>(32, ((total + blocks - 1) / blocks + 31) / 32 * 32)));
+    };
+    s.res_cluster = total <= RES_CLUSTER_GROUPS;
+    const int most = s.res_cluster ? RES_CLUSTER : sms;
+    s.res_groups = groups_of(most);
+    s.res_blocks = s.res_cluster ? RES_CLUSTER : int(std::min<long long>(sms, (total + s.res_groups - 1) / s.res_groups));
+    const size_t smem = res_smem(g);
+    const int rc = with_resident(s.cid_bytes, s.res_cluster, [&](auto kern) -> int {
+        FG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(size_t(res_pad(RES_MAX_AXES + 9)) * 48)));
+        if (s.res_cluster) FG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        FG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 3 * s.res_groups, smem));
+        return FG_OK;
+    });
+    if (rc) return rc;
+    if (per < 1) return FG_OK;
+    s.resident = true;
+    return FG_OK;
+}
+
+// `k` steps (at most RES_MAX_STEPS) as one cooperative launch on the session's stream.
+int launch_resident(Session& s, uint64_t k, std::string& err) {
+    const Geom& g = s.geom;
+    // the set the steps so far left the fields in, and the one this call must leave them in
+    const int from = s.fused ? int(s.steps & 1) : 0, to = s.fused ? int((s.steps + k) & 1) : 0;
+    float *es[2] = {s.e, s.e2}, *hs[2] = {s.h, s.h2}, *ps[2] = {s.psi, s.psi_h2};
+    ResArgs a{};
+    a.g = g;
+    a.node_class = s.node_class;
+    a.classes = s.classes;
+    a.e_src = es[from];
+    a.h_src = hs[from];
+    a.psi_h_src = ps[from];
+    a.e = es[to];
+    a.h = hs[to];
+    a.psi_h = ps[to];
+    a.psi_e = s.psi;
+    a.k_mu = s.sc.k_mu;
+    a.neg0 = -0.0f;
+    a.steps = int(k);
+    a.counter = s.counter;
+    a.bar = s.res_bar;
+    a.error = s.error;
+    a.wait_ns = s.wait_ns;
+    const unsigned q = unsigned(g.n2 + 3) / 4;
+    a.quads = FastDiv(q);
+    a.rows = FastDiv(unsigned(g.n1));
+    const unsigned pass = unsigned(s.res_blocks) * unsigned(s.res_groups);
+    a.drow = pass / q;
+    a.dq = pass % q;
+    a.di = a.drow / unsigned(g.n1);
+    a.dj = a.drow % unsigned(g.n1);
+    a.debye_f = s.debye_f;
+    a.debye_dd = s.debye_dd;
+    a.debye_cb = s.debye_cb;
+    a.debye_table = s.debye_table;
+    a.debye_old = s.debye_old;
+    a.debye_state = s.debye_state;
+    a.n_debye = s.n_debye;
+    a.src = s.sources;
+    a.ind = s.inductors;
+    a.probes = s.probes;
+    a.pe = s.port_edges;
+    a.lp = s.loops;
+    a.series = s.series;
+    a.ns = s.n_sources;
+    a.ni = s.n_inductors;
+    a.n_ports = s.n_ports;
+    a.sc = s.sc;
+    a.plane_k = s.plane_k;
+    a.plane = s.plane_len ? s.plane : nullptr;
+    a.patch = s.patch;
+    a.ntff = s.ntff_len ? s.ntff : nullptr;
+    a.n_patches = s.n_patches;
+    a.design = s.design;
+    a.n_design = s.design_in_steps ? s.n_design : 0;
+    a.hist_base = s.hist_base;
+    a.hist_cap = s.hist_cap;
+    a.hist_e = s.hist_e;
+    a.hist_s = s.hist_s;
+    if (!s.res_cluster) FG_CUDA(cudaMemsetAsync(s.res_bar, 0, sizeof(unsigned), s.stream));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(s.res_blocks));
+    cfg.blockDim = dim3(unsigned(3 * s.res_groups));
+    cfg.dynamicSmemBytes = res_smem(g);
+    cfg.stream = s.stream;
+    cudaLaunchAttribute at[1];
+    if (s.res_cluster) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = unsigned(s.res_blocks);
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return with_resident(s.cid_bytes, s.res_cluster, [&](auto kern) -> int {
+        FG_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+        return FG_OK;
+    });
 }
 
 uint64_t count_launches(const Session& s) {
@@ -1314,6 +1455,11 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     // first, then H; per field the two z slabs (components 0 and 1, derivative along k) first and
     // adjacent, each slab 128-byte aligned, z-slab rows padded to pw slots
     g.pw = int((2 * sim.pml + 3) & ~size_t(3));
+    g.pk = int((n2 + 3) & ~size_t(3));
+    // the k axis as the device keeps it: on grids small enough to step resident, with its layer's slots
+    // numbered by 4-node groups where that is possible
+    std::vector<AxisNode> kax_node = sim.ax[2].node;
+    s->k_quads = (long long)nn <= RES_MAX_NODES && n0 + n1 + n2 <= size_t(RES_MAX_AXES) && res_k_slots(kax_node, sim.pml, g.pw);
     long long psi_total = 0, psi_hbase = 0;
     for (int e = 0; e < 2; ++e) {
         if (e == 1) psi_hbase = psi_total;
@@ -1322,7 +1468,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
         for (const auto& ca : order) {
             g.psi_off[e * 9 + ca[0] * 3 + ca[1]] = psi_total;
             if (sim.pml > 0) {
-                size_t m[3] = {n0, n1, n2};
+                size_t m[3] = {n0, n1, size_t(g.pk)};
                 m[ca[1]] = ca[1] == 2 ? size_t(g.pw) : 2 * sim.pml;
                 psi_total += (long long)((m[0] * m[1] * m[2] + 31) & ~size_t(31));
             }
@@ -1552,6 +1698,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     need += carve_size(std::max<size_t>(t_dft.size(), 1) * 4) * 2;
     need += carve_size(ENERGY_BLOCKS * 8);
     need += carve_size(64);
+    need += carve_size(64);
     const size_t local_tables = cp.blocks.size() * LOCAL_CLASSES * 6;
     if (s->local) need += carve_size(nnp) + carve_size(local_tables * 4);
     need += carve_size(64);
@@ -1625,6 +1772,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     sc.far = d_far;
     s->partial = carve<double>(cur, ENERGY_BLOCKS);
     s->error = carve<int>(cur, 16);
+    s->res_bar = carve<unsigned>(cur, 16);
     if (s->local) {
         s->local_ids = carve<uint8_t>(cur, nnp);
         s->tables = carve<float>(cur, local_tables);
@@ -1691,7 +1839,8 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     FG_CUDA(cudaMemcpyAsync(s->classes, dcls.data(), ncls * sizeof(DevCoef), cudaMemcpyHostToDevice, st));
     FG_CUDA(cudaStreamSynchronize(st));
     std::vector<AxisNode> axes;
-    for (int a = 0; a < 3; ++a) axes.insert(axes.end(), sim.ax[a].node.begin(), sim.ax[a].node.end());
+    for (int a = 0; a < 2; ++a) axes.insert(axes.end(), sim.ax[a].node.begin(), sim.ax[a].node.end());
+    axes.insert(axes.end(), kax_node.begin(), kax_node.end());
     FG_CUDA(cudaMemcpyAsync(s->axes, axes.data(), axes.size() * sizeof(AxisNode), cudaMemcpyHostToDevice, st));
     g.ax[0] = s->axes;
     g.ax[1] = s->axes + n0;
@@ -1699,7 +1848,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     {
         std::vector<float> kv(10 * n2);
         for (size_t k = 0; k < n2; ++k) {
-            const AxisNode& a = sim.ax[2].node[k];
+            const AxisNode& a = kax_node[k];
             const float f[8] = {a.inv_d, a.inv_dd, a.raw_inv_d, a.raw_inv_dd, a.be, a.ce, a.bh, a.ch};
             for (int q = 0; q < 8; ++q) kv[q * n2 + k] = f[q];
             std::memcpy(&kv[8 * n2 + k], &a.slot_e, 4);
@@ -1970,6 +2119,21 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
         *out = s.release();
         return FG_OK;
     }
+    {
+        // resident stepping, unless a pipeline is asked for by name (FIELDGRID_RESIDENT=0 rules it out)
+        const char* rv = std::getenv("FIELDGRID_RESIDENT");
+        const char* nv = std::getenv("FIELDGRID_NO_TMA");
+        if (!(rv && rv[0] == '0') && !(nv && nv[0] == '1') && !std::getenv("FIELDGRID_STEP_DEPTH") && !s->fold &&
+            s->stall_plane < 0 && s->n_wires == 0 && s->n_sheets == 0) {
+            rc = plan_resident(*s, err);
+            if (rc) { session_free(s.release()); return rc; }
+        }
+        if (s->resident) {
+            s->variant += "; steps run resident, " + std::to_string(s->res_blocks) + " blocks";
+            *out = s.release();
+            return FG_OK;
+        }
+    }
     if (s->fused && (s->plane_len || s->ntff_len) && s->n_wires == 0 && s->n_sheets == 0) {
         FG_CUDA(cudaStreamCreateWithFlags(&s->aux, cudaStreamNonBlocking));
         for (int p = 0; p < 2; ++p) {
@@ -2062,9 +2226,19 @@ int session_reset(Session* s, std::string& err) {
 }
 
 int session_step(Session* s, uint64_t k, std::string& err) {
-    if (!s->slots && !s->graph_one[0]) { err = "this session steps only as part of a batch"; return FG_ERR_INVALID; }
+    if (!s->slots && !s->resident && !s->graph_one[0]) { err = "this session steps only as part of a batch"; return FG_ERR_INVALID; }
     FG_CUDA(cudaSetDevice(s->gpu->device));
     uint64_t done = 0;
+    if (s->resident) {
+        while (done < k) {
+            const uint64_t m = std::min<uint64_t>(k - done, RES_MAX_STEPS);
+            const int rc = launch_resident(*s, m, err);
+            if (rc) return rc;
+            done += m;
+            s->steps += m;
+        }
+        return FG_OK;
+    }
     if (s->slots) {
         // 48 steps (24 double steps) keep the phase t mod 6 of the sets, slots and parity
         while (done < k) {
@@ -2163,7 +2337,16 @@ int session_read(Session* s, const std::string& which, float* dst, uint64_t len,
         uint64_t n = std::min<uint64_t>(s->steps, s->sc.cap) * uint64_t(s->sc.ports) * 2;
         return copy(s->series, n);
     }
-    if (which == "plane") return copy(s->plane, s->plane_len);
+    if (which == "plane") {   // the device keeps (frequency, value) major; the record is node major (cpu.rs:336-361)
+        if (s->plane_len > len) { err = "destination too small for plane"; return FG_ERR_INVALID; }
+        std::vector<float> t(s->plane_len);
+        if (s->plane_len) FG_CUDA(cudaMemcpy(t.data(), s->plane, s->plane_len * 4, cudaMemcpyDeviceToHost));
+        s->d2h_bytes += s->plane_len * 4;
+        const uint64_t P = uint64_t(s->geom.n0) * uint64_t(s->geom.n1), per = uint64_t(s->sc.nf) * 10;
+        for (uint64_t q = 0; q < P && s->plane_len; ++q)
+            for (uint64_t m = 0; m < per; ++m) dst[q * per + m] = t[m * P + q];
+        return FG_OK;
+    }
     if (which == "ntff") {
         // the device keeps (frequency, value) major; the record is patch major (cpu.rs:363-415)
         if (s->ntff_len > len) { err = "destination too small for ntff"; return FG_ERR_INVALID; }

@@ -15,14 +15,15 @@ namespace fg {
 // (n2 rounded up to 32, so rows start 128-byte aligned and TMA strides are legal): the device
 // node index is (i*n1 + j)*p2 + k. Fields are component-major with component stride cs
 // (>= n0*n1*p2). The psi slabs follow the reference's layout (sim.rs:659-665), except that a
-// z slab (derivative along k) pads its rows of 2 pml slots to pw, a multiple of 4, so its rows
-// are whole 16-byte units for the TMA; slabs start 128-byte aligned, and each field's two z
+// z slab (derivative along k) pads its rows of 2 pml slots to pw and the x and y slabs theirs of n2
+// nodes to pk, multiples of 4, so rows are whole 16-byte units for the TMA and for 4-node loads; slabs start 128-byte aligned, and each field's two z
 // slabs sit next to each other (one box brings both components).
 struct Geom {
     int n0, n1, n2;
     int p2;
     int pml;
     int pw;                     // z-slab row pitch: 2 pml rounded up to 4
+    int pk;                     // x- and y-slab row pitch: n2 rounded up to 4 (rows of whole 16-byte units)
     long long nn;               // real nodes n0*n1*n2
     long long cs;
     const AxisNode* ax[3];
@@ -65,9 +66,27 @@ struct StepConst {          // per-run scalars (run.rs:433-464 Params)
 };
 
 __device__ __forceinline__ long long psi_at(const Geom& g, int a, int i, int j, int k, int s) {
-    if (a == 0) return ((long long)s * g.n1 + j) * g.n2 + k;
-    if (a == 1) return ((long long)i * (2 * g.pml) + s) * g.n2 + k;
+    if (a == 0) return ((long long)s * g.n1 + j) * g.pk + k;
+    if (a == 1) return ((long long)i * (2 * g.pml) + s) * g.pk + k;
     return ((long long)i * g.n1 + j) * g.pw + s;
+}
+
+// The curl term S^n of one design edge (comp, i, j, k) with the step's new H and E psi (the psi
+// terms are those the E update added; cpu.rs:125-162).
+__device__ __forceinline__ float design_curl(const Geom& g, const int4 d, const float* h, const float* psi) {
+    const int c = d.x;
+    const int p[3] = {d.y, d.z, d.w};
+    const int U = (c + 1) % 3, V = (c + 2) % 3;
+    const long long st[3] = {(long long)g.n1 * g.p2, g.p2, 1};
+    const long long id = ((long long)p[0] * g.n1 + p[1]) * g.p2 + p[2];
+    const float a = h[V * g.cs + id] - h[V * g.cs + id - st[U]];
+    const float b = h[U * g.cs + id] - h[U * g.cs + id - st[V]];
+    const AxisNode& au = g.ax[U][p[U]];
+    const AxisNode& av = g.ax[V][p[V]];
+    float t1 = a * au.inv_dd, t2 = b * av.inv_dd;
+    if (au.slot_e >= 0) t1 += psi[g.psi_off[c * 3 + U] + psi_at(g, U, p[0], p[1], p[2], au.slot_e)];
+    if (av.slot_e >= 0) t2 += psi[g.psi_off[c * 3 + V] + psi_at(g, V, p[0], p[1], p[2], av.slot_e)];
+    return t1 - t2;
 }
 
 // The step index n of the running step: the first kernel of step n raised the counter to n + 1.
@@ -333,7 +352,8 @@ __global__ void k_lumped_probe(const DevSource* __restrict__ src, int ns, DevInd
 }
 
 // cpu.rs:336-361: running DFT of Ex, Ey, Ez (at (n+1) dt) and Hx, Hy (at (n+1/2) dt) on the
-// z-plane k = plane_k; phases formed in f32 like the CPU path.
+// z-plane k = plane_k; phases formed in f32 like the CPU path. Accumulator (frequency k, value c of
+// 10) of node q at acc[(k * 10 + c) * n0 * n1 + q], so a warp's sums coalesce (read back node-major).
 __global__ void k_field_dft(Geom g, int plane_k, StepConst sc, const unsigned* __restrict__ counter, int parity,
                             const float* __restrict__ e, const float* __restrict__ h, float* __restrict__ acc) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -342,8 +362,9 @@ __global__ void k_field_dft(Geom g, int plane_k, StepConst sc, const unsigned* _
     const float te = (float(n) + 1.0f) * sc.dt, th = (float(n) + 0.5f) * sc.dt;
     const long long id = q * g.p2 + plane_k;
     const float f[5] = {e[id], e[g.cs + id], e[2 * g.cs + id], h[id], h[g.cs + id]};
-    float* out = acc + q * sc.nf * 10;
+    const long long pts = (long long)g.n0 * g.n1;
     for (int k = 0; k < sc.nf; ++k) {
+        float* out = acc + (long long)k * 10 * pts + q;
         const float w = sc.omega[k];
         float ce0, ce1, ch0, ch1;
         if (n < sc.cap) {
@@ -356,8 +377,8 @@ __global__ void k_field_dft(Geom g, int plane_k, StepConst sc, const unsigned* _
 #pragma unroll
         for (int c = 0; c < 5; ++c) {
             const float p0 = c >= 3 ? ch0 : ce0, p1 = c >= 3 ? ch1 : ce1;
-            out[k * 10 + 2 * c] += f[c] * p0;
-            out[k * 10 + 2 * c + 1] += f[c] * p1;
+            out[(2 * c) * pts] += f[c] * p0;
+            out[(2 * c + 1) * pts] += f[c] * p1;
         }
     }
 }

@@ -1,0 +1,565 @@
+// Many time steps in one launch, for grids whose state stays in L2: a cooperative kernel with the
+// whole grid's blocks resident steps E and H in place, half a step at a time, with a grid-wide
+// barrier between the halves (two per step; a third where Debye edges or a design history follow the
+// E half).
+//
+// The march kernels move each field once per step through HBM, but a march is a chain of planes: a
+// small grid leaves most SMs idle behind it (65^3: 42 blocks, 33 us a step). In place, a half step
+// has no order inside it, so every 4-node group of the grid is one thread's own work, and the fields
+// (24 B per node) and psi stay in the 126 MB L2 from step to step; a step then costs its L2 traffic
+// (72 B per node) and two barriers instead of three to six kernel launches.
+//
+// Phase A of step n: new H from E (psi of H included); the records that read E after step n - 1
+// (port voltages, running DFTs of E, the NTFF box's M); each Debye edge's and design edge's E^n.
+// Phase B: new E from H, the source and the inductors on the edges of the block's own nodes; the
+// records that read H^n+1/2 (port currents, DFTs of H, the box's J). E does not change in phase A nor
+// H in phase B, so each record reads a settled field without a barrier of its own.
+// Phase C (only with Debye edges or a design history): the Debye ADE and the design edges' curl terms.
+//
+// The arithmetic and its order are those of the other pipelines (cpu.rs:48-167, :239-265, :291-415),
+// so the fields equal theirs bit for bit. A launch of an odd number of steps writes its first step
+// to the other buffer set, so that the latest set stays the one the parity of the step count names.
+#pragma once
+
+#include <vector>
+
+#include "kernels.cuh"
+#include "stencil_tma.cuh"
+
+namespace fg {
+
+// n / d for n < 2^31 by one 64-bit product.
+struct FastDiv {
+    unsigned d = 1, s = 0;
+    unsigned long long m = 1;
+    __host__ __device__ FastDiv() {}
+    __host__ explicit FastDiv(unsigned div) : d(div) {
+        while ((1ull << s) < div) ++s;
+        m = ((1ull << (32 + s)) + div - 1) / div;
+    }
+    __device__ __forceinline__ unsigned operator()(unsigned n) const {
+        return unsigned(((unsigned long long)n * m) >> (32 + s));
+    }
+};
+
+struct ResArgs {
+    Geom g;
+    const void* node_class;
+    const DevCoef* classes;
+    const float *e_src, *h_src, *psi_h_src;   // what the first step reads
+    float *e, *h, *psi_h, *psi_e;             // what every step writes, and all but the first read
+    float k_mu;
+    float neg0;                               // -0.0f (f2::mul's addend)
+    int steps;
+    unsigned* counter;                        // the steps done before the launch
+    unsigned* bar;                            // the grid barrier's arrivals, 0 at launch
+    int* error;
+    unsigned long long wait_ns;
+    FastDiv quads, rows;                      // 4-node groups per row; rows per plane
+    unsigned dq, drow, dj, di;                // a pass of the launch over its groups, as rows and groups; its rows as planes and rows
+    // Debye edges
+    const long long* debye_f;
+    const float *debye_dd, *debye_cb, *debye_table;
+    float *debye_old, *debye_state;
+    int n_debye;
+    // source, inductors, ports
+    const DevSource* src;
+    DevInductor* ind;
+    const DevProbe* probes;
+    const DevPortEdge* pe;
+    const DevLoop* lp;
+    float* series;
+    int ns, ni, n_ports;
+    StepConst sc;
+    // records
+    int plane_k;
+    float* plane;                             // null: none
+    const unsigned* patch;
+    float* ntff;
+    int n_patches;
+    // the design history
+    const int4* design;
+    int n_design;
+    const long long* hist_base;
+    int hist_cap;
+    float *hist_e, *hist_s;
+};
+
+constexpr int RES_GROUPS = 320;             // 4-node groups a block takes at a time, at most
+constexpr int RES_THREADS = 3 * RES_GROUPS;   // a thread per group and component
+constexpr int RES_CLUSTER = 16;             // blocks of a launch on the smallest grids: one cluster
+constexpr int RES_MAX_AXES = 1536;   // nodes of the three axes together (their factors sit in shared memory)
+
+__host__ __device__ inline int res_pad(int n) { return (n + 3) & ~3; }
+
+// The axes' factors in shared memory, 12 words per node: along i and j as ResNode records (a row's
+// factors in two 16-byte loads), along k as 12 arrays (length padded to 4 with zeros; a group's four in
+// one load): inv_d, inv_dd, raw_d, raw_dd, be, ce, bh, ch, then per group the first slot of a group that
+// reaches the layer, or -1 (its nodes' slots follow one another, see res_k_slots). The CPML's b and c are
+// zero outside the layer.
+struct __align__(16) ResHalf {   // of the H or the E update
+    float inv;
+    int slot;
+    float raw, b;
+};
+struct __align__(16) ResNode {
+    ResHalf f[2];                // H, E
+    float c[2];
+    float pad[2];
+};
+
+// Numbers the layer's slots along k so that the nodes of a 4-node group (k a multiple of 4) that lie in
+// the layer have consecutive slots from a multiple of 4 on: the low layer's slots are its nodes, the
+// high layer's start past them at its first group. pw becomes the slots' row pitch. False, and nothing
+// changed, where one group would hold nodes of both layers or the pitch would outgrow the march's
+// staged boxes.
+inline bool res_k_slots(std::vector<AxisNode>& ax, size_t pml, int& pw) {
+    const int n = int(ax.size()), p = int(pml);
+    if (p == 0 || n <= 2 * p + 2) return true;   // no layer: no slots
+    const int low = res_pad(p), high = (n - 1 - p) & ~3, w = low + res_pad(n) - high;
+    if (high < low || (w > 32 && pw <= 32)) return false;
+    for (int k = 0; k < n; ++k)
+        for (int* s : {&ax[size_t(k)].slot_e, &ax[size_t(k)].slot_h})
+            if (*s >= 0) *s = k < p ? k : low + (k - high);
+    pw = w;
+    return true;
+}
+inline size_t res_smem(const Geom& g) { return size_t(res_pad(g.n0) + res_pad(g.n1) + res_pad(g.n2)) * 12 * 4; }
+
+__device__ __forceinline__ void res_fill_rows(ResNode* t, int n, const AxisNode* ax) {
+    for (int q = threadIdx.x; q < n; q += blockDim.x) {
+        const AxisNode v = ax[q];
+        ResNode r;
+        r.f[0] = ResHalf{v.inv_d, v.slot_h, v.raw_inv_d, v.bh};
+        r.f[1] = ResHalf{v.inv_dd, v.slot_e, v.raw_inv_dd, v.be};
+        r.c[0] = v.ch;
+        r.c[1] = v.ce;
+        r.pad[0] = r.pad[1] = 0.f;
+        t[q] = r;
+    }
+}
+
+// E's factors at node 0 are cleared: no edge there updates along k, and its psi stays 0.
+__device__ __forceinline__ void res_fill_k(float* z, int n, const AxisNode* ax) {
+    const int np = res_pad(n);
+    int* slot = reinterpret_cast<int*>(z + 8 * np);
+    for (int q = threadIdx.x; q < np; q += blockDim.x) {
+        AxisNode v{0, 0, 0, 0, 0, 0, 0, 0, -1, -1};
+        if (q < n) v = ax[q];
+        const bool le = v.slot_e >= 0 && q > 0, lh = v.slot_h >= 0;
+        const float f[8] = {v.inv_d, v.inv_dd, v.raw_inv_d, v.raw_inv_dd, le ? v.be : 0.f, le ? v.ce : 0.f,
+                            lh ? v.bh : 0.f, lh ? v.ch : 0.f};
+#pragma unroll
+        for (int t = 0; t < 8; ++t) z[t * np + q] = f[t];
+        if (q < np / 4) {
+            int first = -1;   // any live node's slot less its place in the group
+            for (int t = 0; t < 4 && 4 * q + t < n; ++t) {
+                const int e = ax[4 * q + t].slot_e, h = ax[4 * q + t].slot_h;
+                if (e >= 0) first = e - t;
+                else if (h >= 0) first = h - t;
+            }
+            slot[q] = first;
+        }
+    }
+}
+
+// Every block of the launch arrives and waits for all: of a launch that is one cluster by the cluster's
+// hardware barrier, else through a counter in global memory; false when the wait ran out (the error word
+// is set, and every block leaves at this barrier or the next). The block's writes before it are
+// visible to all after it.
+template <bool CLUSTER>
+__device__ __forceinline__ bool res_barrier(const ResArgs& a, unsigned target) {
+    if constexpr (CLUSTER) {
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return true;
+    }
+    __syncthreads();
+    int bad = 0;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+        unsigned v;
+        unsigned long long t0 = 0;
+        for (unsigned spin = 0;; ++spin) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+            if (v >= target) break;
+            if ((spin & 255u) == 255u) {
+                unsigned long long t;
+                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+                if (t0 == 0) t0 = t;
+                else if (t - t0 > a.wait_ns) {
+                    atomicExch(a.error, 3);
+                    bad = 1;
+                    break;
+                }
+            }
+        }
+    }
+    return !__syncthreads_or(bad);
+}
+
+// Four nodes along k as two packed pairs (f2's operations round each lane as the scalar ones do).
+struct Quad {
+    float2 a, b;
+};
+__device__ __forceinline__ Quad ld4(const float* p) {
+    const float4 f = *reinterpret_cast<const float4*>(p);
+    return Quad{make_float2(f.x, f.y), make_float2(f.z, f.w)};
+}
+__device__ __forceinline__ void st4(float* p, const Quad& q) {
+    *reinterpret_cast<float4*>(p) = make_float4(q.a.x, q.a.y, q.b.x, q.b.y);
+}
+__device__ __forceinline__ Quad q_zero() { return Quad{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
+__device__ __forceinline__ Quad q_bc(float v) { return Quad{make_float2(v, v), make_float2(v, v)}; }
+__device__ __forceinline__ Quad operator+(const Quad& x, const Quad& y) { return Quad{f2::add(x.a, y.a), f2::add(x.b, y.b)}; }
+__device__ __forceinline__ Quad operator-(const Quad& x, const Quad& y) { return Quad{f2::sub(x.a, y.a), f2::sub(x.b, y.b)}; }
+__device__ __forceinline__ Quad q_mul(const Quad& x, const Quad& y, float2 z) { return Quad{f2::mul(x.a, y.a, z), f2::mul(x.b, y.b, z)}; }
+// the values one node up (the fourth from `next`) or one node down (the first from `prev`)
+__device__ __forceinline__ Quad q_up(const Quad& x, float next) { return Quad{make_float2(x.a.y, x.b.x), make_float2(x.b.y, next)}; }
+__device__ __forceinline__ Quad q_down(const Quad& x, float prev) { return Quad{make_float2(prev, x.a.x), make_float2(x.a.y, x.b.x)}; }
+// one CPML term, psi' = b psi + (c d) raw (cpu.rs:73-99): psi becomes psi', t gains it
+__device__ __forceinline__ void q_psi(Quad& t, Quad& psi, const Quad& d, const Quad& b, const Quad& c, const Quad& raw, float2 z) {
+    psi = q_mul(b, psi, z) + q_mul(q_mul(c, d, z), raw, z);
+    t = t + psi;
+}
+
+// The class ids of 4 nodes in one load.
+template <typename CID>
+__device__ __forceinline__ uint4 res_ids(const CID* p) {
+    if constexpr (sizeof(CID) == 1) {
+        const unsigned v = __ldg(reinterpret_cast<const unsigned*>(p));
+        return make_uint4(v & 255u, v >> 8 & 255u, v >> 16 & 255u, v >> 24);
+    } else if constexpr (sizeof(CID) == 2) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+        return make_uint4(v.x & 65535u, v.x >> 16, v.y & 65535u, v.y >> 16);
+    } else {
+        return __ldg(reinterpret_cast<const uint4*>(p));
+    }
+}
+
+// One component C of the field (F = 1: E from H, F = 0: H from E) on the 4 nodes from (i, j, k)
+// (cpu.rs:48-167): its two curl terms R - S, R the difference along i or j that its row decides (x: j,
+// y and z: i), S the other (along k for the x and y components, along j for z), with the sign of the y
+// component's pair turned (R - S = -(S - R) exactly).
+//
+// A node whose update does not run keeps its value by a select; its psi is advanced all the same where
+// the layer covers it: such a psi is read by no update (its edge never runs), and it stays 0 where the
+// reference's does by the cleared factors. Every field load comes before the first store.
+template <int C, int F, typename CID>
+__device__ __forceinline__ void res_update(const ResArgs& a, const ResNode* X, const ResNode* Y, const float* Z, int np2, unsigned row,
+                                           int i, int j, int k, const float* src, const float* own, float* out,
+                                           const float* psi_in, float* psi_out) {
+    const Geom& g = a.g;
+    const unsigned id = row * unsigned(g.p2) + unsigned(k), cs = unsigned(g.cs);
+    const float2 z = make_float2(a.neg0, a.neg0);
+    constexpr bool ALONG_I = C != 0, S_J = C == 2;    // R's axis; S along j (else along k)
+    const unsigned sj = unsigned(g.p2), si = unsigned(g.n1) * sj, sr = ALONG_I ? si : sj;
+    const bool has_i = F ? i > 0 : i + 1 < g.n0, has_j = F ? j > 0 : j + 1 < g.n1;
+    const unsigned ido = unsigned(C) * cs + id;
+    const Quad f = ld4(own + ido);
+    if (!(ALONG_I ? has_i : has_j) || (S_J && !has_j)) {   // no neighbour along R or S: nothing to update
+        if (out != own) st4(out + ido, f);
+        return;
+    }
+    const unsigned idr = (C == 2 ? cs : 2 * cs) + id, ids = (C == 0 ? cs : 0u) + id;
+    const Quad r0 = ld4(src + idr), r1 = ld4(src + (F ? idr - sr : idr + sr));
+    const Quad s0 = ld4(src + ids);
+    const int nk = g.n2 - k;
+    Quad s1;
+    if constexpr (S_J) s1 = ld4(src + (F ? ids - sj : ids + sj));
+    else if constexpr (F) s1 = q_down(s0, k > 0 ? src[ids - 1] : 0.f);
+    else s1 = q_up(s0, nk > 4 ? src[ids + 4] : 0.f);
+    const ResNode* tr = ALONG_I ? X + i : Y + j;
+    const ResHalf fr = tr->f[F];
+    float2 ca0, ca1, cb0, cb1;
+    if constexpr (F) {
+        const uint4 cid = res_ids(static_cast<const CID*>(a.node_class) + id);
+        const float* t = reinterpret_cast<const float*>(a.classes) + C;
+        const float fa = __ldg(t + cid.x * 8), fb = __ldg(t + cid.x * 8 + 4);   // most groups hold one class
+        ca0 = ca1 = make_float2(fa, fa);
+        cb0 = cb1 = make_float2(fb, fb);
+        if (cid.y != cid.x || cid.z != cid.x || cid.w != cid.x) {
+            ca0.y = __ldg(t + cid.y * 8); cb0.y = __ldg(t + cid.y * 8 + 4);
+            ca1 = make_float2(__ldg(t + cid.z * 8), __ldg(t + cid.w * 8));
+            cb1 = make_float2(__ldg(t + cid.z * 8 + 4), __ldg(t + cid.w * 8 + 4));
+        }
+    }
+    const Quad dr = F ? r0 - r1 : r1 - r0, ds = F ? s0 - s1 : s1 - s0;
+    Quad R = q_mul(dr, q_bc(fr.inv), z), S;
+    if (fr.slot >= 0) {
+        const unsigned o = unsigned(g.psi_off[(F ? 0 : 9) + C * 3 + (ALONG_I ? 0 : 1)]) + unsigned(k) +
+                           (ALONG_I ? unsigned(fr.slot) * unsigned(g.n1) + unsigned(j)
+                                    : unsigned(i) * unsigned(2 * g.pml) + unsigned(fr.slot)) * unsigned(g.pk);
+        Quad p = ld4(psi_in + o);
+        q_psi(R, p, dr, q_bc(fr.b), q_bc(tr->c[F]), q_bc(fr.raw), z);
+        st4(psi_out + o, p);
+    }
+    if constexpr (S_J) {
+        const ResHalf fs = Y[j].f[F];
+        S = q_mul(ds, q_bc(fs.inv), z);
+        if (fs.slot >= 0) {
+            const unsigned o = unsigned(g.psi_off[(F ? 0 : 9) + C * 3 + 1]) + unsigned(k) +
+                               (unsigned(i) * unsigned(2 * g.pml) + unsigned(fs.slot)) * unsigned(g.pk);
+            Quad p = ld4(psi_in + o);
+            q_psi(S, p, ds, q_bc(fs.b), q_bc(Y[j].c[F]), q_bc(fs.raw), z);
+            st4(psi_out + o, p);
+        }
+    } else {
+        S = q_mul(ds, ld4(Z + (F ? 1 : 0) * np2 + k), z);
+        const int sl = reinterpret_cast<const int*>(Z + 8 * np2)[k >> 2];
+        if (sl >= 0) {
+            const unsigned o = unsigned(g.psi_off[(F ? 0 : 9) + C * 3 + 2]) + row * unsigned(g.pw) + unsigned(sl);
+            Quad p = ld4(psi_in + o);
+            q_psi(S, p, ds, ld4(Z + (F ? 4 : 6) * np2 + k), ld4(Z + (F ? 5 : 7) * np2 + k), ld4(Z + (F ? 3 : 2) * np2 + k), z);
+            st4(psi_out + o, p);
+        }
+    }
+    const Quad t = C == 1 ? S - R : R - S;
+    Quad n;
+    if constexpr (F) {
+        n = q_mul(Quad{ca0, ca1}, f, z) + q_mul(Quad{cb0, cb1}, t, z);
+        n.a = f2::pick(cb0.x != 0.f && (S_J || k > 0), cb0.y != 0.f, n.a, f.a);
+        n.b = f2::pick(cb1.x != 0.f, cb1.y != 0.f, n.b, f.b);
+    } else {
+        n = f - q_mul(q_bc(a.k_mu), t, z);
+        if (!S_J) {   // the row's last node has no k + 1 neighbour (the padding past it is 0 and stays 0)
+            n.a = f2::pick(nk > 1, nk > 2, n.a, f.a);
+            n.b = f2::pick(nk > 3, nk > 4, n.b, f.b);
+        }
+    }
+    st4(out + ido, n);
+}
+
+// A warp's share of a half step: component C of the groups from `first` on, `stride` groups apart.
+template <int C, int F, typename CID>
+__device__ __forceinline__ void res_half(const ResArgs& a, const ResNode* X, const ResNode* Y, const float* Z, int np2, unsigned first,
+                                         const float* src, const float* own, float* out, const float* psi_in, float* psi_out) {
+    unsigned row = a.quads(first), col = first - row * a.quads.d;
+    unsigned i = a.rows(row), j = row - i * a.rows.d;
+    while (i < unsigned(a.g.n0)) {
+        res_update<C, F, CID>(a, X, Y, Z, np2, row, int(i), int(j), int(col * 4u), src, own, out, psi_in, psi_out);
+        // the next group: the stride as (planes, rows, groups)
+        col += a.dq;
+        row += a.drow;
+        j += a.dj;
+        i += a.di;
+        if (col >= a.quads.d) { col -= a.quads.d; ++row; ++j; }
+        if (j >= a.rows.d) { j -= a.rows.d; ++i; }
+    }
+}
+
+template <int F, typename CID>
+__device__ __forceinline__ void res_field(const ResArgs& a, int comp, const ResNode* X, const ResNode* Y, const float* Z, int np2,
+                                          unsigned first, const float* src, const float* own, float* out, const float* psi_in,
+                                          float* psi_out) {
+    if (comp == 0) res_half<0, F, CID>(a, X, Y, Z, np2, first, src, own, out, psi_in, psi_out);
+    else if (comp == 1) res_half<1, F, CID>(a, X, Y, Z, np2, first, src, own, out, psi_in, psi_out);
+    else res_half<2, F, CID>(a, X, Y, Z, np2, first, src, own, out, psi_in, psi_out);
+}
+
+// A port's voltage (F = 0, E settled after step n) or current (F = 1, H of step n) into its series
+// entry: one warp, the f64 sums of probe_block (the same order for up to 32 edges).
+template <int F>
+__device__ __forceinline__ void res_probe(const ResArgs& a, int port, unsigned n) {
+    const DevProbe d = a.probes[port];
+    const int lane = threadIdx.x & 31;
+    double s = 0.0;
+    if (F == 0) {
+        for (int q = lane; q < d.count; q += 32) {
+            const DevPortEdge x = a.pe[d.first + q];
+            s -= double(a.e[(long long)d.comp * a.g.cs + x.id] * x.w);
+        }
+    } else {
+        for (int q = lane; q < d.loop_count; q += 32) {
+            const DevLoop x = a.lp[d.loop_first + q];
+            s += double(a.h[x.f] * x.w);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0 && n < a.sc.cap) a.series[((long long)n * a.sc.ports + port) * 2 + F] = float(s);
+}
+
+// The step's DFT phase factors of frequency k: (E's cos, sin, H's cos, sin) dt; sign -1 as the plane
+// DFT forms them beyond the tables, +1 as the NTFF does (f32, cpu.rs:344-353, :403-405).
+__device__ __forceinline__ float4 res_phase(const StepConst& sc, const float* table, unsigned n, int k, bool far) {
+    if (n < sc.cap) return *reinterpret_cast<const float4*>(table + ((long long)n * sc.nf + k) * 4);
+    const float w = sc.omega[k], te = (float(n) + 1.0f) * sc.dt, th = (float(n) + 0.5f) * sc.dt;
+    if (far) return make_float4(cosf(-w * te) * sc.dt, sinf(-w * te) * sc.dt, cosf(-w * th) * sc.dt, sinf(-w * th) * sc.dt);
+    return make_float4(cosf(w * te) * sc.dt, -sinf(w * te) * sc.dt, cosf(w * th) * sc.dt, -sinf(w * th) * sc.dt);
+}
+
+// k_field_dft's sums over E (F = 0) or H (F = 1) of step n.
+template <int F>
+__device__ __forceinline__ void res_plane(const ResArgs& a, unsigned n, unsigned t, unsigned nt) {
+    const Geom& g = a.g;
+    const unsigned pts = unsigned(g.n0) * unsigned(g.n1);
+    constexpr int NC = F ? 2 : 3, C0 = F ? 3 : 0;
+    const float* src = F ? a.h : a.e;
+    for (unsigned q = t; q < pts; q += nt) {
+        const long long id = (long long)q * g.p2 + a.plane_k;
+        float f[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) f[c] = src[c * g.cs + id];
+        for (int k = 0; k < a.sc.nf; ++k) {
+            const float4 ph = res_phase(a.sc, a.sc.dft, n, k, false);
+            const float p0 = F ? ph.z : ph.x, p1 = F ? ph.w : ph.y;
+            float* out = a.plane + ((long long)k * 10 + 2 * C0) * pts + q;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                out[(2 * c) * (long long)pts] += f[c] * p0;
+                out[(2 * c + 1) * (long long)pts] += f[c] * p1;
+            }
+        }
+    }
+}
+
+// k_ntff's sums: M from E (F = 0) or J from H (F = 1) of step n.
+template <int F>
+__device__ __forceinline__ void res_ntff(const ResArgs& a, unsigned n, unsigned t, unsigned nt) {
+    const long long cs = a.g.cs;
+    const int P = a.n_patches;
+    for (unsigned p = t; p < unsigned(P); p += nt) {
+        const unsigned meta = a.patch[p];
+        const int axis = meta & 3;
+        const float side = (meta & 4) ? 1.0f : -1.0f;
+        const int u = (axis + 1) % 3, v = (axis + 2) % 3;
+        auto at = [&](int m) { return a.patch[(long long)m * P + p]; };
+        float f[3] = {0, 0, 0}, nrm[3] = {0, 0, 0}, o[3];
+        nrm[axis] = side;
+        if (F == 0) {
+            f[u] = 0.5f * (a.e[u * cs + at(1)] + a.e[u * cs + at(2)]);
+            f[v] = 0.5f * (a.e[v * cs + at(3)] + a.e[v * cs + at(4)]);
+            o[0] = f[1] * nrm[2] - f[2] * nrm[1];
+            o[1] = f[2] * nrm[0] - f[0] * nrm[2];
+            o[2] = f[0] * nrm[1] - f[1] * nrm[0];
+        } else {
+            f[u] = 0.25f * (a.h[u * cs + at(5)] + a.h[u * cs + at(6)] + a.h[u * cs + at(7)] + a.h[u * cs + at(8)]);
+            f[v] = 0.25f * (a.h[v * cs + at(9)] + a.h[v * cs + at(10)] + a.h[v * cs + at(11)] + a.h[v * cs + at(12)]);
+            o[0] = nrm[1] * f[2] - nrm[2] * f[1];
+            o[1] = nrm[2] * f[0] - nrm[0] * f[2];
+            o[2] = nrm[0] * f[1] - nrm[1] * f[0];
+        }
+        for (int k = 0; k < a.sc.nf; ++k) {
+            const float4 ph = res_phase(a.sc, a.sc.far, n, k, true);
+            const float p0 = F ? ph.z : ph.x, p1 = F ? ph.w : ph.y;
+            float* acc = a.ntff + ((long long)k * 12 + (F ? 0 : 6)) * P + p;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                acc[(long long)(2 * c) * P] += p0 * o[c];
+                acc[(long long)(2 * c + 1) * P] += p1 * o[c];
+            }
+        }
+    }
+}
+
+// The block that updates the node of field index f.
+__device__ __forceinline__ unsigned res_block_of(const ResArgs& a, long long f, unsigned blocks, unsigned groups) {
+    const long long id = f % a.g.cs;
+    return ((unsigned(id / a.g.p2) * a.quads.d + unsigned(id % a.g.p2) / 4u) / groups) % blocks;
+}
+
+// At most one block per SM, every block resident: a cooperative launch. The blocks take the grid's
+// 4-node groups, in row order, a third of its threads' number at a time in turn, three warps (one per
+// component) to 32 groups: a block's groups are whole rows (its j neighbours and the three components' shared loads are
+// mostly in its L1), and the layer's heavier groups fall on all blocks alike.
+template <typename CID, bool CLUSTER>
+__global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_constant__ ResArgs a) {
+    extern __shared__ __align__(16) float res_sm[];
+    const Geom& g = a.g;
+    const int np2 = res_pad(g.n2);
+    ResNode *X = reinterpret_cast<ResNode*>(res_sm), *Y = X + res_pad(g.n0);
+    float* Z = reinterpret_cast<float*>(Y + res_pad(g.n1));
+    res_fill_rows(X, g.n0, g.ax[0]);
+    res_fill_rows(Y, g.n1, g.ax[1]);
+    res_fill_k(Z, g.n2, g.ax[2]);
+    const int w = threadIdx.x >> 5, comp = w % 3;                                      // the warp's component
+    const unsigned groups = blockDim.x / 3u;
+    const unsigned first = blockIdx.x * groups + unsigned(w / 3) * 32u + (threadIdx.x & 31u);   // the lane's first group
+    const unsigned G = gridDim.x, b = blockIdx.x;
+    // the lists are shared out 32 entries at a time, one warp of every block before a block's next
+    const unsigned t = (unsigned(w) * G + b) * 32u + (threadIdx.x & 31u), nt = G * blockDim.x;
+    const unsigned n0 = *(volatile const unsigned*)a.counter;
+    int own = 0;   // a source or inductor edge among the block's nodes
+    for (int q = threadIdx.x; q < a.ns; q += blockDim.x) own |= res_block_of(a, a.src[q].f, G, groups) == b;
+    for (int q = threadIdx.x; q < a.ni; q += blockDim.x) own |= res_block_of(a, a.ind[q].f, G, groups) == b;
+    own = __syncthreads_or(own);
+    const bool third = a.n_debye > 0 || a.n_design > 0;
+    const long long hist0 = a.n_design ? *a.hist_base : 0;
+    unsigned target = 0;
+    for (int s = 0; s <= a.steps; ++s) {
+        const unsigned n = n0 + unsigned(s);
+        // ---- phase A: what reads E^n (E after step n - 1) ...
+        if (s > 0) {
+            if (threadIdx.x < 32)
+                for (int p = int(G - 1 - b); p < a.n_ports; p += int(G)) res_probe<0>(a, p, n - 1);
+            if (a.plane) res_plane<0>(a, n - 1, t, nt);
+            if (a.ntff) res_ntff<0>(a, n - 1, t, nt);
+        }
+        if (s == a.steps) break;
+        const float* e_in = s ? a.e : a.e_src;
+        long long slot = -1;   // this step's place in the design history
+        if (a.n_design) {
+            slot = (long long)n - hist0;
+            if (slot >= a.hist_cap) slot = -1;
+        }
+        for (int q = int(t); q < a.n_debye; q += int(nt)) a.debye_old[q] = e_in[a.debye_f[q]];
+        if (slot >= 0)
+            for (int q = int(t); q < a.n_design; q += int(nt)) {
+                const int4 d = a.design[q];
+                a.hist_e[slot * a.n_design + q] = e_in[d.x * g.cs + ((long long)d.y * g.n1 + d.z) * g.p2 + d.w];
+            }
+        // ... and the new H
+        const float *h_in = s ? a.h : a.h_src, *p_in = s ? a.psi_h : a.psi_h_src;
+        res_field<0, CID>(a, comp, X, Y, Z, np2, first, e_in, h_in, a.h, p_in, a.psi_h);
+        if (!res_barrier<CLUSTER>(a, target += G)) return;
+        // ---- phase B: what reads the new H, and the new E
+        if (threadIdx.x < 32)
+            for (int p = int(G - 1 - b); p < a.n_ports; p += int(G)) res_probe<1>(a, p, n);
+        if (a.plane) res_plane<1>(a, n, t, nt);
+        if (a.ntff) res_ntff<1>(a, n, t, nt);
+        res_field<1, CID>(a, comp, X, Y, Z, np2, first, a.h, e_in, a.e, a.psi_e, a.psi_e);
+        if (own) {   // the source, then the inductors (lumped_block), on the block's own edges
+            __syncthreads();
+            const float p = n < a.sc.cap ? a.sc.pulse[n] : pulse_at(a.sc, (float(n) + 0.5f) * a.sc.dt);
+            for (int q = threadIdx.x; q < a.ns; q += blockDim.x) {
+                const DevSource x = a.src[q];
+                if (res_block_of(a, x.f, G, groups) == b) a.e[x.f] -= x.src * p;
+            }
+            __syncthreads();
+            for (int q = threadIdx.x; q < a.ni; q += blockDim.x) {
+                const DevInductor d = a.ind[q];
+                if (res_block_of(a, d.f, G, groups) == b) {
+                    const float x = a.e[d.f] - d.ke * d.cur;
+                    a.e[d.f] = x;
+                    a.ind[q].cur = d.cur + d.ki * x;
+                }
+            }
+        }
+        if (!res_barrier<CLUSTER>(a, target += G)) return;
+        if (third) {
+            // ---- phase C: the Debye ADE (k_debye_post_cb; its edges carry no source or element) and
+            // the design edges' curl terms (k_design_record)
+            const int poles = a.n_debye ? int(a.debye_table[0]) : 0;
+            for (int q = int(t); q < a.n_debye; q += int(nt)) {
+                const long long fi = a.debye_f[q];
+                float s0 = 0.0f;
+                for (int k = 0; k < poles; ++k)
+                    s0 += 0.5f * (1.0f + a.debye_table[1 + 2 * k]) * a.debye_state[(long long)k * a.n_debye + q];
+                const float next = a.e[fi] - a.debye_cb[q] * s0;
+                a.e[fi] = next;
+                const float de = next - a.debye_old[q], w = a.debye_dd[q];
+                for (int k = 0; k < poles; ++k) {
+                    const long long p = (long long)k * a.n_debye + q;
+                    a.debye_state[p] = a.debye_table[1 + 2 * k] * a.debye_state[p] + w * a.debye_table[2 + 2 * k] * de;
+                }
+            }
+            if (slot >= 0)
+                for (int q = int(t); q < a.n_design; q += int(nt))
+                    a.hist_s[slot * a.n_design + q] = design_curl(g, a.design[q], a.h, a.psi_e);
+            if (!res_barrier<CLUSTER>(a, target += G)) return;
+        }
+    }
+    if (t == 0) *a.counter = n0 + unsigned(a.steps);
+}
+
+}  // namespace fg

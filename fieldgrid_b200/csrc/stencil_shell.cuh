@@ -104,8 +104,8 @@ __device__ __forceinline__ void shell_h_row(const Geom& g, const ShellRows& b, c
     const long long row = ((long long)i * g.n1 + j) * g.p2;
     const long long si = (long long)g.n1 * g.p2, sj = g.p2;
     // psi offsets of this row in the x and y slabs (psi_idx, sim.rs:659-665); the z slab per node
-    const long long px = ai.slot_h >= 0 ? ((long long)ai.slot_h * g.n1 + j) * g.n2 : 0;
-    const long long py = aj.slot_h >= 0 ? ((long long)i * (2 * g.pml) + aj.slot_h) * g.n2 : 0;
+    const long long px = ai.slot_h >= 0 ? ((long long)ai.slot_h * g.n1 + j) * g.pk : 0;
+    const long long py = aj.slot_h >= 0 ? ((long long)i * (2 * g.pml) + aj.slot_h) * g.pk : 0;
     const long long pz = ((long long)i * g.n1 + j) * g.pw;
     for (int q = int(threadIdx.x & 31); q < len; q += 32) {
         const int k = strips && q >= b.za ? b.zb + (q - b.za) : q;
@@ -171,8 +171,8 @@ __device__ __forceinline__ void shell_e_row(const Geom& g, const ShellRows& b, c
     const long long cs = g.cs;
     const long long row = ((long long)i * g.n1 + j) * g.p2;
     const long long si = (long long)g.n1 * g.p2, sj = g.p2;
-    const long long px = ai.slot_e >= 0 ? ((long long)ai.slot_e * g.n1 + j) * g.n2 : 0;
-    const long long py = aj.slot_e >= 0 ? ((long long)i * (2 * g.pml) + aj.slot_e) * g.n2 : 0;
+    const long long px = ai.slot_e >= 0 ? ((long long)ai.slot_e * g.n1 + j) * g.pk : 0;
+    const long long py = aj.slot_e >= 0 ? ((long long)i * (2 * g.pml) + aj.slot_e) * g.pk : 0;
     const long long pz = ((long long)i * g.n1 + j) * g.pw;
     for (int q = int(threadIdx.x & 31); q < len; q += 32) {
         const int k = strips && q >= b.za ? b.zb + (q - b.za) : q;
