@@ -134,6 +134,9 @@ struct FluxJob {
     std::vector<int4> edges;
     uint64_t N = 0, L = 0, S = 0;
     bool ckpt = false, sep = false;
+    bool resident = false;    // the sweep as resident launches (adjoint_resident.cuh)
+    int* dwin = nullptr;      // of its Debye edges on the flux plane
+    uint8_t* wmask = nullptr;
     Session* s = nullptr;
     size_t fbytes = 0, pbytes = 0, nd_s = 0, dbytes = 0;
     struct Ck { float *e = nullptr, *h = nullptr, *psi = nullptr, *deb = nullptr; };
@@ -161,6 +164,8 @@ struct FluxJob {
         for (cudaEvent_t e : evs) cudaEventDestroy(e);
         if (sw) cudaStreamDestroy(sw);
         for (float* p : {lE[0], lE[1], lH[0], lH[1], lpsi[0], lpsi[1], dw, cam, cbm, lds, lold}) cudaFree(p);
+        cudaFree(dwin);
+        cudaFree(wmask);
         cudaFree(ga);
         cudaFree(gb);
         cudaFree(ck_mem);
@@ -178,6 +183,16 @@ struct FluxJob {
         k_adj_set<<<1, 1, 0, s->stream>>>(s->hist_base, b, s->counter, cnt, counter ? 1 : 0);
         FG_CUDA(cudaGetLastError());
         return FG_OK;
+    }
+
+    // Whether every step's design history takes no more device memory than the checkpoints asked for
+    // and their ring of two segments: then it is kept and no segment runs twice (160x160x96 cells, 27,720
+    // design edges, 640 steps: 142 MB against 10 checkpoints of 78 MB; the re-runs were half the
+    // backward's device time).
+    bool keep_history() const {
+        const size_t p2 = (sim->n[2] + 31) & ~size_t(31), cs = (sim->n[0] * sim->n[1] * p2 + 31) & ~size_t(31);
+        const size_t per = 2 * 3 * cs * 4 + sim->debye_edges.size() * sim->poles.size() * 4;   // without its psi
+        return uint64_t(N) * info.size() * 8 <= per * S + 2 * L * info.size() * 8;
     }
 
     // checks, the session, the checkpoints and the adjoint buffers
@@ -213,6 +228,7 @@ struct FluxJob {
         res.segment_len = L;
         res.design_edges = info.size();
         sep = sp.transposes == 1;
+        if (want_grad && S > 1 && keep_history()) { L = N; S = 1; }
 
         RunSpec rs;
         rs.driven = driven;
@@ -250,13 +266,29 @@ struct FluxJob {
         wi = sp.win_hi[0] - sp.win_lo[0];
         wj = sp.win_hi[1] - sp.win_lo[1];
         const int nd = int(edges.size());
-        for (auto** p : {&lE[0], &lE[1], &lH[0]}) FG_CUDA(cudaMalloc(p, fbytes));
+        // a stored history and a grid that steps resident: the sweep in place, one set of everything
+        resident = s->resident && !sep && !ckpt;
+        for (auto** p : {&lE[0], &lH[0]}) FG_CUDA(cudaMalloc(p, fbytes));
+        FG_CUDA(cudaMalloc(&lpsi[0], pbytes));
         if (sep) {
             for (auto** p : {&cam, &cbm}) FG_CUDA(cudaMalloc(p, fbytes));
-        } else {
+        } else if (!resident) {
             FG_CUDA(cudaMalloc(&lH[1], fbytes));
         }
-        for (auto** p : {&lpsi[0], &lpsi[1]}) FG_CUDA(cudaMalloc(p, pbytes));
+        if (!resident) {
+            FG_CUDA(cudaMalloc(&lE[1], fbytes));
+            FG_CUDA(cudaMalloc(&lpsi[1], pbytes));
+        } else {
+            FG_CUDA(cudaMalloc(&dwin, std::max<size_t>(size_t(s->n_debye), 1) * 4));
+            FG_CUDA(cudaMalloc(&wmask, (wi * wj + 3) & ~size_t(3)));
+            const int ra = with_adj_resident(s->cid_bytes, s->res_cluster, [&](auto kern) -> int {
+                FG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             int(size_t(res_pad(RES_MAX_AXES + 9)) * 32)));
+                if (s->res_cluster) FG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+                return FG_OK;
+            });
+            if (ra) return ra;
+        }
         FG_CUDA(cudaMalloc(&lds, dbytes));
         FG_CUDA(cudaMalloc(&lold, std::max<size_t>(size_t(s->n_debye), 1) * 4));
         FG_CUDA(cudaMalloc(&dw, std::max<size_t>(wi * wj * 8, 1) * 4));
@@ -381,10 +413,12 @@ struct FluxJob {
         b0 = std::chrono::steady_clock::now();
         for (float* p : {lE[0], lE[1], lH[0], lH[1]})
             if (p) FG_CUDA(cudaMemsetAsync(p, 0, fbytes, st));
-        for (float* p : {lpsi[0], lpsi[1]}) FG_CUDA(cudaMemsetAsync(p, 0, pbytes, st));
+        for (float* p : {lpsi[0], lpsi[1]})
+            if (p) FG_CUDA(cudaMemsetAsync(p, 0, pbytes, st));
         FG_CUDA(cudaMemsetAsync(lds, 0, dbytes, st));
         FG_CUDA(cudaMemsetAsync(ga, 0, size_t(std::max(nd, 1)) * 8, st));
         FG_CUDA(cudaMemsetAsync(gb, 0, size_t(std::max(nd, 1)) * 8, st));
+        if (resident) return sweep_resident();
         if (sep) {
             const dim3 blk(64, 4, 1), grd((g.n2 + 63) / 64, (g.n1 + 3) / 4, g.n0);
             switch (s->cid_bytes) {
@@ -494,12 +528,67 @@ struct FluxJob {
         return FG_OK;
     }
 
+    // the whole sweep as resident launches on the sweep's stream (the buffers are cleared on st)
+    int sweep_resident() {
+        const Geom& g = s->geom;
+        cudaStream_t st = s->stream;
+        AdjResArgs A{};
+        resident_shape(*s, A.r);
+        A.r.e = lE[0];
+        A.r.h = lH[0];
+        A.psi = lpsi[0];
+        A.plane_k = int(sp.plane_k);
+        A.i0 = int(sp.win_lo[0]);
+        A.wi = int(wi);
+        A.j0 = int(sp.win_lo[1]);
+        A.wj = int(wj);
+        A.w = dw;
+        A.dft = s->sc.dft;
+        A.r.design = s->design;
+        A.r.n_design = int(edges.size());
+        A.hist_e = s->hist_e;
+        A.hist_s = s->hist_s;
+        A.ga = ga;
+        A.gb = gb;
+        A.ls = lds;
+        A.lold = lold;
+        A.dwin = dwin;
+        A.wmask = wmask;
+        A.n_hi = (long long)N;
+        FG_CUDA(cudaMemsetAsync(lold, 0, std::max<size_t>(size_t(s->n_debye), 1) * 4, st));
+        FG_CUDA(cudaMemsetAsync(wmask, 0, (wi * wj + 3) & ~size_t(3), st));
+        if (s->n_debye)
+            k_adj_debye_window<<<unsigned((s->n_debye + 255) / 256), 256, 0, st>>>(
+                s->debye_f, s->n_debye, g, A.plane_k, A.i0, A.wi, A.j0, A.wj, dwin, reinterpret_cast<unsigned*>(wmask));
+        k_adj_source_e<<<unsigned((wi * wj + 127) / 128), 128, 0, st>>>(A);
+        FG_CUDA(cudaGetLastError());
+        cudaEvent_t e0, e1;
+        int rc;
+        if ((rc = event(&e0, true)) || (rc = event(&e1, true))) return rc;
+        FG_CUDA(cudaEventRecord(e0, st));
+        for (uint64_t left = N; left > 0;) {
+            A.r.steps = int(std::min<uint64_t>(left, RES_MAX_STEPS));
+            A.n_hi = (long long)left;
+            rc = with_adj_resident(s->cid_bytes, s->res_cluster, [&](auto kern) -> int {
+                return launch_res(*s, kern, A, adj_res_smem(g), st, err);
+            });
+            if (rc) return rc;
+            left -= uint64_t(A.r.steps);
+        }
+        FG_CUDA(cudaEventRecord(e1, st));
+        t_sw.push_back({e0, e1});
+        return FG_OK;
+    }
+
     // waits for the backward; the parts' times and the chain rule to the design voxels
     int finish() {
         FG_CUDA(cudaSetDevice(gpu->device));
         FG_CUDA(cudaStreamSynchronize(sw));
         FG_CUDA(cudaStreamSynchronize(s->stream));
         res.backward_ms = ms_since(b0);
+        int flag = 0;
+        FG_CUDA(cudaMemcpy(&flag, s->error, sizeof(int), cudaMemcpyDeviceToHost));
+        if (flag) { err = "a bounded wait in the fused step ran out (code " + std::to_string(flag) + ")"; return FG_ERR_CUDA; }
         for (auto& pr : t_rec) { float x = 0; FG_CUDA(cudaEventElapsedTime(&x, pr.first, pr.second)); res.recompute_ms += x; }
         for (auto& pr : t_sw) { float x = 0; FG_CUDA(cudaEventElapsedTime(&x, pr.first, pr.second)); res.adjoint_ms += x; }
         const int nd = int(edges.size());

@@ -27,6 +27,7 @@
 #include "stencil_resident.cuh"
 #include "setup_kernels.cuh"
 #include "adjoint_kernels.cuh"
+#include "adjoint_resident.cuh"
 
 #include <cudaTypedefs.h>
 #include <cub/cub.cuh>
@@ -734,6 +735,13 @@ int with_resident(int cid_bytes, bool cluster, F&& f) {
 }
 
 // Whether a session's steps run resident, and its launch shape.
+template <typename F>
+int with_adj_resident(int cid_bytes, bool cluster, F&& f) {
+    if (cid_bytes == 1) return cluster ? f(k_adj_resident<uint8_t, true>) : f(k_adj_resident<uint8_t, false>);
+    if (cid_bytes == 2) return cluster ? f(k_adj_resident<uint16_t, true>) : f(k_adj_resident<uint16_t, false>);
+    return cluster ? f(k_adj_resident<uint32_t, true>) : f(k_adj_resident<uint32_t, false>);
+}
+
 int plan_resident(Session& s, std::string& err) {
     const Geom& g = s.geom;
     s.resident = false;
@@ -764,34 +772,20 @@ int plan_resident(Session& s, std::string& err) {
     return FG_OK;
 }
 
-// `k` steps (at most RES_MAX_STEPS) as one cooperative launch on the session's stream.
-int launch_resident(Session& s, uint64_t k, std::string& err) {
+// The launch shape and index arithmetic shared by the resident kernels of a session.
+void resident_shape(const Session& s, ResArgs& a) {
     const Geom& g = s.geom;
-    // the set the steps so far left the fields in, and the one this call must leave them in
-    const int from = s.fused ? int(s.steps & 1) : 0, to = s.fused ? int((s.steps + k) & 1) : 0;
-    float *es[2] = {s.e, s.e2}, *hs[2] = {s.h, s.h2}, *ps[2] = {s.psi, s.psi_h2};
-    ResArgs a{};
     a.g = g;
     a.node_class = s.node_class;
     a.classes = s.classes;
-    a.e_src = es[from];
-    a.h_src = hs[from];
-    a.psi_h_src = ps[from];
-    a.e = es[to];
-    a.h = hs[to];
-    a.psi_h = ps[to];
-    a.psi_e = s.psi;
     a.k_mu = s.sc.k_mu;
     a.neg0 = -0.0f;
-    a.steps = int(k);
-    a.counter = s.counter;
     a.bar = s.res_bar;
     a.error = s.error;
     a.wait_ns = s.wait_ns;
-    const unsigned q = unsigned(g.n2 + 3) / 4;
+    const unsigned q = unsigned(g.n2 + 3) / 4, pass = unsigned(s.res_blocks) * unsigned(s.res_groups);
     a.quads = FastDiv(q);
     a.rows = FastDiv(unsigned(g.n1));
-    const unsigned pass = unsigned(s.res_blocks) * unsigned(s.res_groups);
     a.drow = pass / q;
     a.dq = pass % q;
     a.di = a.drow / unsigned(g.n1);
@@ -800,9 +794,52 @@ int launch_resident(Session& s, uint64_t k, std::string& err) {
     a.debye_dd = s.debye_dd;
     a.debye_cb = s.debye_cb;
     a.debye_table = s.debye_table;
+    a.n_debye = s.n_debye;
+}
+
+// Launches a resident kernel on `st` with every block resident: one cluster, or a cooperative launch.
+template <typename K, typename A>
+int launch_res(const Session& s, K kern, const A& a, size_t smem, cudaStream_t st, std::string& err) {
+    if (!s.res_cluster) FG_CUDA(cudaMemsetAsync(s.res_bar, 0, sizeof(unsigned), st));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(s.res_blocks));
+    cfg.blockDim = dim3(unsigned(3 * s.res_groups));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    if (s.res_cluster) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = unsigned(s.res_blocks);
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    FG_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+    return FG_OK;
+}
+
+// `k` steps (at most RES_MAX_STEPS) as one cooperative launch on the session's stream.
+int launch_resident(Session& s, uint64_t k, std::string& err) {
+    const Geom& g = s.geom;
+    // the set the steps so far left the fields in, and the one this call must leave them in
+    const int from = s.fused ? int(s.steps & 1) : 0, to = s.fused ? int((s.steps + k) & 1) : 0;
+    float *es[2] = {s.e, s.e2}, *hs[2] = {s.h, s.h2}, *ps[2] = {s.psi, s.psi_h2};
+    ResArgs a{};
+    resident_shape(s, a);
+    a.e_src = es[from];
+    a.h_src = hs[from];
+    a.psi_h_src = ps[from];
+    a.e = es[to];
+    a.h = hs[to];
+    a.psi_h = ps[to];
+    a.psi_e = s.psi;
+    a.steps = int(k);
+    a.counter = s.counter;
     a.debye_old = s.debye_old;
     a.debye_state = s.debye_state;
-    a.n_debye = s.n_debye;
     a.src = s.sources;
     a.ind = s.inductors;
     a.probes = s.probes;
@@ -824,26 +861,8 @@ int launch_resident(Session& s, uint64_t k, std::string& err) {
     a.hist_cap = s.hist_cap;
     a.hist_e = s.hist_e;
     a.hist_s = s.hist_s;
-    if (!s.res_cluster) FG_CUDA(cudaMemsetAsync(s.res_bar, 0, sizeof(unsigned), s.stream));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(unsigned(s.res_blocks));
-    cfg.blockDim = dim3(unsigned(3 * s.res_groups));
-    cfg.dynamicSmemBytes = res_smem(g);
-    cfg.stream = s.stream;
-    cudaLaunchAttribute at[1];
-    if (s.res_cluster) {
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = unsigned(s.res_blocks);
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    } else {
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-    }
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
     return with_resident(s.cid_bytes, s.res_cluster, [&](auto kern) -> int {
-        FG_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
-        return FG_OK;
+        return launch_res(s, kern, a, res_smem(g), s.stream, err);
     });
 }
 
