@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -46,6 +47,10 @@ RunSpec run_spec(uint64_t driven, const fg_pulse* pulse, const fg_extras* x) {
 struct Far {
     std::vector<double> pos, area, jm;  // jm: 12 doubles per patch (J then M, re/im, x y z)
     double freq = 0;
+    // the device layouts of this far field's patches, and the calls using them one at a time
+    mutable std::vector<FarDevice*> devices;
+    mutable std::mutex lock;
+    ~Far() { for (FarDevice* d : devices) far_device_free(d); }
 };
 
 // FIELDGRID_SETUP_TIMES=1: fg_run prints the wall time of its phases to stderr
@@ -466,7 +471,8 @@ int fg_far_field(fg_gpu* g, const fg_far* f, const double* dirs, uint64_t n, dou
     if (!f || (n && (!dirs || !out))) return FG_ERR_INVALID;
     if (g) {
         std::string e;
-        int rc = far_field_gpu(g->g, f->f.pos.data(), f->f.area.data(), f->f.jm.data(), f->f.area.size(), f->f.freq,
+        std::lock_guard<std::mutex> hold(f->f.lock);
+        int rc = far_field_gpu(g->g, f->f.devices, f->f.pos.data(), f->f.area.data(), f->f.jm.data(), f->f.area.size(), f->f.freq,
                                dirs, n, out, e);
         if (rc) g_last_error = e;
         return rc;

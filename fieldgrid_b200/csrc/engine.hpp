@@ -85,9 +85,13 @@ int session_kernel_times(Session* s, uint64_t steps, std::vector<std::pair<std::
 uint64_t session_h2d_bytes(const Session* s);
 uint64_t session_d2h_bytes(const Session* s);
 
-// Far field on the device: fields for n directions (6 doubles each).
-int far_field_gpu(Gpu* g, const double* pos, const double* area, const double* jm, uint64_t count, double freq,
-                  const double* dirs, uint64_t n, double* out, std::string& err);
+// Far field on the device: fields for n directions (6 doubles each). `devices` keeps what a far-field
+// handle has laid out on each device (far_device_free gives it back); the caller keeps calls on one
+// handle from running at the same time.
+struct FarDevice;
+void far_device_free(FarDevice* d);
+int far_field_gpu(Gpu* g, std::vector<FarDevice*>& devices, const double* pos, const double* area, const double* jm,
+                  uint64_t count, double freq, const double* dirs, uint64_t n, double* out, std::string& err);
 
 int sim_try_new(const struct fg_sim_spec* spec, HostSim** out, std::string& err);
 
