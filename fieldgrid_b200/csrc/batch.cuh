@@ -16,6 +16,12 @@
 // launches above: seven launches per step for the whole batch, with each grid's arithmetic that of
 // its own TMA step.
 //
+// Resident mode (tile 6): where every grid's state fits the L2, each grid steps on its own, many steps in
+// one resident launch (stencil_resident.cuh) before the next grid's: its fields stay in the L2 over those
+// steps, where the other modes carry every grid's fields through HBM each step. blocks_per_sm launches
+// run side by side, so that one grid's barriers hide behind another's work. Calls of few steps go
+// through the graphs of the fastest other mode.
+//
 // The autotuner times a few steps of each candidate (tile shape, blocks per SM of the persistent
 // launch, planes per item; graph branches; the merged launches) on the real batch, keeps the
 // fastest, resets every grid to step 0 and captures the graphs with it.
@@ -132,6 +138,8 @@ struct BatchShape {
 constexpr int BATCH_BRANCHES = 3;          // graph branches, each grid's own step (TMA march + shell)
 constexpr int BATCH_BRANCHES_DIRECT = 4;   // graph branches with the direct-load fused march
 constexpr int BATCH_MERGED = 5;            // one TMA march and one shell launch over all grids
+constexpr int BATCH_RESIDENT = 6;          // each grid's steps as resident launches
+constexpr uint64_t BATCH_RESIDENT_STEPS = 8;   // a call's steps at least to go that way
 
 constexpr int BATCH_TILES[3][2] = {{32, 8}, {64, 4}, {32, 4}};
 
@@ -166,7 +174,39 @@ struct Batch {
     int* d_shell_block = nullptr;      // per shell block: its grid
     int shell_blocks = 0;
     std::vector<int> merged_rest;      // grids the merged launches leave to their own direct-load march
+    // resident mode: the launches that share the SMs (0: off); the graphs keep `shape` for short calls
+    int share = 0;
+    bool resident_ok = false;
 };
+
+// Plans every grid's resident launches for `share` of them side by side; false when a grid cannot.
+int batch_plan_resident(Batch& B, int share, std::string& err) {
+    B.resident_ok = true;
+    for (Session* s : B.s) {
+        if (!resident_allowed(*s)) { B.resident_ok = false; return FG_OK; }
+        const int rc = plan_resident(*s, share, err);
+        if (rc) return rc;
+        if (!s->resident) { B.resident_ok = false; return FG_OK; }
+    }
+    return FG_OK;
+}
+
+// `k` steps (at most RES_MAX_STEPS) of every grid as resident launches on the grids' streams, between the
+// batch stream's earlier and later work. The launches go to `share` streams in turn.
+int batch_resident(Batch& B, uint64_t k, std::string& err) {
+    FG_CUDA(cudaEventRecord(B.fork, B.stream));
+    const size_t lanes = std::min<size_t>(size_t(std::max(B.share, 1)), B.s.size());
+    for (size_t b = 0; b < lanes; ++b) FG_CUDA(cudaStreamWaitEvent(B.s[b]->stream, B.fork, 0));
+    for (size_t b = 0; b < B.s.size(); ++b) {
+        const int rc = launch_resident(*B.s[b], k, err, B.s[b % lanes]->stream);
+        if (rc) return rc;
+    }
+    for (size_t b = 0; b < lanes; ++b) {
+        FG_CUDA(cudaEventRecord(B.join[b], B.s[b]->stream));
+        FG_CUDA(cudaStreamWaitEvent(B.stream, B.join[b], 0));
+    }
+    return FG_OK;
+}
 
 constexpr auto batch_tma_local =
     k_batch_tma<TMA_TJ, TMA_TK, uint8_t, TMA_SHAPES[0].stages, TMA_SEGMAX, true, TMA_SHAPES[0].minb>;
@@ -483,6 +523,15 @@ int batch_step(Batch& B, uint64_t k, std::string& err) {
     uint64_t done = 0;
     while (done < k) {
         const int parity = int(B.steps & 1);
+        if (B.share > 0 && k - done >= BATCH_RESIDENT_STEPS) {
+            const uint64_t m = std::min<uint64_t>(k - done, RES_MAX_STEPS);
+            const int rc = batch_resident(B, m, err);
+            if (rc) return rc;
+            done += m;
+            B.steps += m;
+            for (Session* s : B.s) s->steps = B.steps;
+            continue;
+        }
         if (parity == 0 && k - done >= uint64_t(B.graph_steps) && B.graph_many) {
             FG_CUDA(cudaGraphLaunch(B.graph_many, B.stream));
             done += B.graph_steps;
@@ -573,6 +622,13 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
     if (rc) return rc;
     // the tuner: each candidate runs a warm-up step then a timed block of steps from the live state
     BatchShape best = fixed;
+    int share = 0;
+    if (!tune && fixed.tile == BATCH_RESIDENT) {
+        share = std::min(std::max(fixed.blocks_per_sm, 1), 4);
+        if ((rc = batch_plan_resident(*B, share, err))) return rc;
+        if (!B->resident_ok) { err = "a grid of this batch does not step resident"; return FG_ERR_INVALID; }
+        best = BatchShape{BATCH_BRANCHES, 0, 0};
+    }
     if (tune) {
         cudaEvent_t e0, e1;
         FG_CUDA(cudaEventCreate(&e0));
@@ -602,6 +658,22 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
             B->trials.push_back({sh, ms / timed});
             if (ms / timed < best_ms) { best_ms = ms / timed; best = sh; }
         }
+        for (int sh = 1; sh <= 3 && !rc; ++sh) {   // resident launches, `sh` side by side
+            const uint64_t many = 2 * BATCH_RESIDENT_STEPS;
+            if ((rc = batch_plan_resident(*B, sh, err)) || !B->resident_ok) break;
+            B->share = sh;
+            for (int pass = 0; pass < 2 && !rc; ++pass) {   // a warm-up, then the timed one
+                FG_CUDA(cudaEventRecord(e0, B->stream));
+                rc = batch_resident(*B, many, err);
+                FG_CUDA(cudaEventRecord(e1, B->stream));
+                FG_CUDA(cudaEventSynchronize(e1));
+            }
+            float ms = 0;
+            if (!rc) FG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+            B->trials.push_back({BatchShape{BATCH_RESIDENT, sh, 0}, ms / float(many)});
+            if (!rc && ms / float(many) < best_ms) { best_ms = ms / float(many); share = sh; }
+        }
+        B->share = 0;
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         if (rc) return rc;
@@ -616,6 +688,11 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
         if ((rc = batch_reset(*B, err))) return rc;
     }
     if ((rc = batch_apply_shape(*B, best, err))) return rc;
+    if (share > 0) {
+        if ((rc = batch_plan_resident(*B, share, err))) return rc;
+        B->share = share;
+        B->persistent_blocks = B->s[0]->res_blocks;
+    }
     B->graph_steps = std::max(2, graph_steps + (graph_steps & 1));
     if ((rc = batch_capture(*B, B->graph_steps, 0, &B->graph_many, err))) return rc;
     if ((rc = batch_capture(*B, 1, 0, &B->graph_one[0], err))) return rc;
@@ -627,7 +704,7 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
 int batch_new_c(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vector<RunSpec>& specs, bool tune,
                 int tile, int blocks_per_sm, int seg, int graph_steps, Batch** out, std::string& err) {
     BatchShape sh;
-    sh.tile = std::min(std::max(tile, 0), BATCH_MERGED);
+    sh.tile = std::min(std::max(tile, 0), BATCH_RESIDENT);
     sh.blocks_per_sm = std::max(blocks_per_sm, 0);
     sh.seg = seg > 0 ? seg : 32;
     return batch_new(gpu, sims, specs, tune, sh, graph_steps > 0 ? graph_steps : 10, out, err);
@@ -648,8 +725,8 @@ int batch_read(Batch& B, uint64_t index, const std::string& which, float* dst, u
 
 void batch_info(const Batch& B, int* tile, int* blocks_per_sm, int* seg, int* persistent_blocks, double* tuned_ms,
                 uint64_t* steps) {
-    if (tile) *tile = B.shape.tile;
-    if (blocks_per_sm) *blocks_per_sm = B.shape.blocks_per_sm;
+    if (tile) *tile = B.share > 0 ? BATCH_RESIDENT : B.shape.tile;
+    if (blocks_per_sm) *blocks_per_sm = B.share > 0 ? B.share : B.shape.blocks_per_sm;
     if (seg) *seg = B.shape.seg;
     if (persistent_blocks) *persistent_blocks = B.persistent_blocks;
     if (tuned_ms) *tuned_ms = B.tuned_ms;

@@ -734,7 +734,17 @@ int with_resident(int cid_bytes, bool cluster, F&& f) {
     return cluster ? f(k_resident<uint32_t, true>) : f(k_resident<uint32_t, false>);
 }
 
-// Whether a session's steps run resident, and its launch shape.
+// Whether a session's steps may run resident: not where a pipeline is asked for by name
+// (FIELDGRID_RESIDENT=0 rules it out), nor with thin wires or resistive sheets.
+bool resident_allowed(const Session& s) {
+    const char* rv = std::getenv("FIELDGRID_RESIDENT");
+    const char* nv = std::getenv("FIELDGRID_NO_TMA");
+    return !(rv && rv[0] == '0') && !(nv && nv[0] == '1') && !std::getenv("FIELDGRID_STEP_DEPTH") && !s.slots && !s.fold &&
+           s.stall_plane < 0 && s.n_wires == 0 && s.n_sheets == 0;
+}
+
+// Whether a session's steps run resident, and its launch shape, with room on each SM for the blocks of
+// `share` such launches (of sessions stepped side by side).
 template <typename F>
 int with_adj_resident(int cid_bytes, bool cluster, F&& f) {
     if (cid_bytes == 1) return cluster ? f(k_adj_resident<uint8_t, true>) : f(k_adj_resident<uint8_t, false>);
@@ -742,7 +752,7 @@ int with_adj_resident(int cid_bytes, bool cluster, F&& f) {
     return cluster ? f(k_adj_resident<uint32_t, true>) : f(k_adj_resident<uint32_t, false>);
 }
 
-int plan_resident(Session& s, std::string& err) {
+int plan_resident(Session& s, int share, std::string& err) {
     const Geom& g = s.geom;
     s.resident = false;
     if (!s.k_quads) return FG_OK;
@@ -752,7 +762,7 @@ int plan_resident(Session& s, std::string& err) {
     if (!coop) return FG_OK;
     const long long total = (long long)g.n0 * g.n1 * ((g.n2 + 3) / 4);
     auto groups_of = [&](long long blocks) {   // per block and pass, in whole warps
-        return int(std::min<long long>(RES_GROUPS, std::max<long long>(32, ((total + blocks - 1) / blocks + 31) / 32 * 32)));
+        return int(std::min<long long>(RES_GROUPS / share / 32 * 32, std::max<long long>(32, ((total + blocks - 1) / blocks + 31) / 32 * 32)));
     };
     s.res_cluster = total <= RES_CLUSTER_GROUPS;
     const int most = s.res_cluster ? RES_CLUSTER : sms;
@@ -821,8 +831,8 @@ int launch_res(const Session& s, K kern, const A& a, size_t smem, cudaStream_t s
     return FG_OK;
 }
 
-// `k` steps (at most RES_MAX_STEPS) as one cooperative launch on the session's stream.
-int launch_resident(Session& s, uint64_t k, std::string& err) {
+// `k` steps (at most RES_MAX_STEPS) as one cooperative launch on the session's stream, or on `st`.
+int launch_resident(Session& s, uint64_t k, std::string& err, cudaStream_t st = nullptr) {
     const Geom& g = s.geom;
     // the set the steps so far left the fields in, and the one this call must leave them in
     const int from = s.fused ? int(s.steps & 1) : 0, to = s.fused ? int((s.steps + k) & 1) : 0;
@@ -862,7 +872,7 @@ int launch_resident(Session& s, uint64_t k, std::string& err) {
     a.hist_e = s.hist_e;
     a.hist_s = s.hist_s;
     return with_resident(s.cid_bytes, s.res_cluster, [&](auto kern) -> int {
-        return launch_res(s, kern, a, res_smem(g), s.stream, err);
+        return launch_res(s, kern, a, res_smem(g), st ? st : s.stream, err);
     });
 }
 
@@ -2139,12 +2149,8 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
         return FG_OK;
     }
     {
-        // resident stepping, unless a pipeline is asked for by name (FIELDGRID_RESIDENT=0 rules it out)
-        const char* rv = std::getenv("FIELDGRID_RESIDENT");
-        const char* nv = std::getenv("FIELDGRID_NO_TMA");
-        if (!(rv && rv[0] == '0') && !(nv && nv[0] == '1') && !std::getenv("FIELDGRID_STEP_DEPTH") && !s->fold &&
-            s->stall_plane < 0 && s->n_wires == 0 && s->n_sheets == 0) {
-            rc = plan_resident(*s, err);
+        if (resident_allowed(*s)) {
+            rc = plan_resident(*s, 1, err);
             if (rc) { session_free(s.release()); return rc; }
         }
         if (s->resident) {
