@@ -383,53 +383,79 @@ __global__ void k_field_dft(Geom g, int plane_k, StepConst sc, const unsigned* _
     }
 }
 
-// cpu.rs:363-415: per NTFF patch, tangential E (2-edge mean) and H (4-edge mean), J = n x H,
-// M = E x n, accumulated with dt e^{-j w t}. Component-major on the device so a warp's loads and
-// stores coalesce: the patch record's word m of patch g at pidx[m * patches + g], accumulator
-// (frequency k, value c of 12) at acc[(k * 12 + c) * patches + g] (read back in the reference's
-// patch-major order).
-__global__ void k_ntff(const unsigned* __restrict__ pidx, int patches, long long cs, StepConst sc,
-                       const unsigned* __restrict__ counter, int parity, const float* __restrict__ e,
-                       const float* __restrict__ h, float* __restrict__ acc) {
+// The tangential currents of one NTFF patch of a face normal to axis A (cpu.rs:363-400): the means of E
+// (two edges) and H (four) along u = A + 1 and v = A + 2, and M = E x n, J = n x H, whose component along A
+// is 0. `word(m)`: the patch record's word m.
+struct NtffM {
+    float u, v;
+};
+template <int A, typename W>
+__device__ __forceinline__ NtffM ntff_m(W word, long long cs, const float* e, float side) {
+    constexpr int U = (A + 1) % 3, V = (A + 2) % 3;
+    const float eu = 0.5f * (e[U * cs + word(1)] + e[U * cs + word(2)]);
+    const float ev = 0.5f * (e[V * cs + word(3)] + e[V * cs + word(4)]);
+    return NtffM{ev * side, -(eu * side)};
+}
+template <int A, typename W>
+__device__ __forceinline__ NtffM ntff_j(W word, long long cs, const float* h, float side) {
+    constexpr int U = (A + 1) % 3, V = (A + 2) % 3;
+    const float hu = 0.25f * (h[U * cs + word(5)] + h[U * cs + word(6)] + h[U * cs + word(7)] + h[U * cs + word(8)]);
+    const float hv = 0.25f * (h[V * cs + word(9)] + h[V * cs + word(10)] + h[V * cs + word(11)] + h[V * cs + word(12)]);
+    return NtffM{-(side * hv), side * hu};
+}
+
+// acc += phase * current for the two components along u and v (values FIRST + 2 c, + 1: re, im).
+template <int A>
+__device__ __forceinline__ void ntff_add(float* acc, long long patches, const NtffM& x, float p0, float p1) {
+    constexpr int U = (A + 1) % 3, V = (A + 2) % 3;
+    float *u = acc + (2 * U) * patches, *v = acc + (2 * V) * patches;
+    const float u0 = u[0], u1 = u[patches], v0 = v[0], v1 = v[patches];
+    u[0] = u0 + p0 * x.u;
+    u[patches] = u1 + p1 * x.u;
+    v[0] = v0 + p0 * x.v;
+    v[patches] = v1 + p1 * x.v;
+}
+
+// The NTFF phase factors of step n and frequency k: E's (re, im), H's (re, im), times dt.
+__device__ __forceinline__ float4 ntff_phase(const StepConst& sc, unsigned n, int k) {
+    if (n < sc.cap) return __ldg(reinterpret_cast<const float4*>(sc.far) + ((long long)n * sc.nf + k));
+    const float te = (float(n) + 1.0f) * sc.dt, th = (float(n) + 0.5f) * sc.dt, w = sc.omega[k];
+    return make_float4(cosf(-w * te) * sc.dt, sinf(-w * te) * sc.dt, cosf(-w * th) * sc.dt, sinf(-w * th) * sc.dt);
+}
+
+template <int A>
+__device__ __forceinline__ void ntff_patch(const unsigned* __restrict__ pidx, int g, int patches, long long cs, const StepConst& sc,
+                                           unsigned n, float side, const float* __restrict__ e, const float* __restrict__ h,
+                                           float* __restrict__ acc) {
+    auto word = [&](int m) { return __ldg(pidx + (long long)m * patches + g); };
+    const NtffM m = ntff_m<A>(word, cs, e, side), j = ntff_j<A>(word, cs, h, side);
+    for (int k = 0; k < sc.nf; ++k) {
+        const float4 p = ntff_phase(sc, n, k);
+        float* o = acc + (long long)k * 12 * patches + g;
+        ntff_add<A>(o, patches, j, p.z, p.w);
+        ntff_add<A>(o + 6ll * patches, patches, m, p.x, p.y);
+    }
+}
+
+// cpu.rs:363-415: per NTFF patch, tangential E and H means, J = n x H, M = E x n, accumulated with
+// dt e^{-j w t}. Component-major on the device so a warp's loads and stores coalesce: the patch record's
+// word m of patch g at pidx[m * patches + g], accumulator (frequency k, value c of 12) at
+// acc[(k * 12 + c) * patches + g] (read back in the reference's patch-major order). One body per face
+// axis: with the axis a run-time index the two fields' components went through local memory and the
+// components along the normal, always 0, were accumulated too:
+// 65 -> 39 us for 195,000 patches at three frequencies.
+__global__ void __launch_bounds__(128) k_ntff(const unsigned* __restrict__ pidx, int patches, long long cs, StepConst sc,
+                                              const unsigned* __restrict__ counter, int parity, const float* __restrict__ e,
+                                              const float* __restrict__ h, float* __restrict__ acc) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= patches) return;
     const unsigned n = step_of(counter, parity);
-    unsigned b[13];
-#pragma unroll
-    for (int m = 0; m < 13; ++m) b[m] = pidx[(long long)m * patches + g];
-    const unsigned meta = b[0];
+    const unsigned meta = pidx[g];
     const int axis = meta & 3;
     const float side = (meta & 4) ? 1.0f : -1.0f;
-    const int u = (axis + 1) % 3, v = (axis + 2) % 3;
-    float ef[3] = {0, 0, 0}, hf[3] = {0, 0, 0};
-    ef[u] = 0.5f * (e[u * cs + b[1]] + e[u * cs + b[2]]);
-    ef[v] = 0.5f * (e[v * cs + b[3]] + e[v * cs + b[4]]);
-    hf[u] = 0.25f * (h[u * cs + b[5]] + h[u * cs + b[6]] + h[u * cs + b[7]] + h[u * cs + b[8]]);
-    hf[v] = 0.25f * (h[v * cs + b[9]] + h[v * cs + b[10]] + h[v * cs + b[11]] + h[v * cs + b[12]]);
-    float nrm[3] = {0, 0, 0};
-    nrm[axis] = side;
-    const float jv[3] = {nrm[1] * hf[2] - nrm[2] * hf[1], nrm[2] * hf[0] - nrm[0] * hf[2], nrm[0] * hf[1] - nrm[1] * hf[0]};
-    const float mv[3] = {ef[1] * nrm[2] - ef[2] * nrm[1], ef[2] * nrm[0] - ef[0] * nrm[2], ef[0] * nrm[1] - ef[1] * nrm[0]};
-    const float te = (float(n) + 1.0f) * sc.dt, th = (float(n) + 0.5f) * sc.dt;
-    for (int k = 0; k < sc.nf; ++k) {
-        const float wf = sc.omega[k];
-        float pe0, pe1, ph0, ph1;
-        if (n < sc.cap) {
-            const float* t = sc.far + ((long long)n * sc.nf + k) * 4;
-            pe0 = t[0]; pe1 = t[1]; ph0 = t[2]; ph1 = t[3];
-        } else {
-            pe0 = cosf(-wf * te) * sc.dt; pe1 = sinf(-wf * te) * sc.dt;
-            ph0 = cosf(-wf * th) * sc.dt; ph1 = sinf(-wf * th) * sc.dt;
-        }
-        float* o = acc + (long long)k * 12 * patches + g;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            o[(long long)(2 * c) * patches] += ph0 * jv[c];
-            o[(long long)(2 * c + 1) * patches] += ph1 * jv[c];
-            o[(long long)(6 + 2 * c) * patches] += pe0 * mv[c];
-            o[(long long)(6 + 2 * c + 1) * patches] += pe1 * mv[c];
-        }
-    }
+    if (axis == 0) ntff_patch<0>(pidx, g, patches, cs, sc, n, side, e, h, acc);
+    else if (axis == 1) ntff_patch<1>(pidx, g, patches, cs, sc, n, side, e, h, acc);
+    else ntff_patch<2>(pidx, g, patches, cs, sc, n, side, e, h, acc);
 }
 
 // cpu.rs:417-421: sum of E^2 + (376.73 H)^2 in f64, one partial per block. Row padding and the

@@ -379,12 +379,10 @@ __device__ __forceinline__ void res_probe(const ResArgs& a, int port, unsigned n
     if (lane == 0 && n < a.sc.cap) a.series[((long long)n * a.sc.ports + port) * 2 + F] = float(s);
 }
 
-// The step's DFT phase factors of frequency k: (E's cos, sin, H's cos, sin) dt; sign -1 as the plane
-// DFT forms them beyond the tables, +1 as the NTFF does (f32, cpu.rs:344-353, :403-405).
-__device__ __forceinline__ float4 res_phase(const StepConst& sc, const float* table, unsigned n, int k, bool far) {
-    if (n < sc.cap) return *reinterpret_cast<const float4*>(table + ((long long)n * sc.nf + k) * 4);
+// The step's plane-DFT phase factors of frequency k: E's (re, im), H's (re, im), times dt (cpu.rs:344-353).
+__device__ __forceinline__ float4 res_phase(const StepConst& sc, unsigned n, int k) {
+    if (n < sc.cap) return __ldg(reinterpret_cast<const float4*>(sc.dft) + ((long long)n * sc.nf + k));
     const float w = sc.omega[k], te = (float(n) + 1.0f) * sc.dt, th = (float(n) + 0.5f) * sc.dt;
-    if (far) return make_float4(cosf(-w * te) * sc.dt, sinf(-w * te) * sc.dt, cosf(-w * th) * sc.dt, sinf(-w * th) * sc.dt);
     return make_float4(cosf(w * te) * sc.dt, -sinf(w * te) * sc.dt, cosf(w * th) * sc.dt, -sinf(w * th) * sc.dt);
 }
 
@@ -401,7 +399,7 @@ __device__ __forceinline__ void res_plane(const ResArgs& a, unsigned n, unsigned
 #pragma unroll
         for (int c = 0; c < NC; ++c) f[c] = src[c * g.cs + id];
         for (int k = 0; k < a.sc.nf; ++k) {
-            const float4 ph = res_phase(a.sc, a.sc.dft, n, k, false);
+            const float4 ph = res_phase(a.sc, n, k);
             const float p0 = F ? ph.z : ph.x, p1 = F ? ph.w : ph.y;
             float* out = a.plane + ((long long)k * 10 + 2 * C0) * pts + q;
 #pragma unroll
@@ -414,41 +412,26 @@ __device__ __forceinline__ void res_plane(const ResArgs& a, unsigned n, unsigned
 }
 
 // k_ntff's sums: M from E (F = 0) or J from H (F = 1) of step n.
+template <int F, int A>
+__device__ __forceinline__ void res_ntff_patch(const ResArgs& a, unsigned n, unsigned p, float side) {
+    const int P = a.n_patches;
+    auto word = [&](int m) { return __ldg(a.patch + (long long)m * P + p); };
+    NtffM x;
+    if constexpr (F) x = ntff_j<A>(word, a.g.cs, a.h, side);
+    else x = ntff_m<A>(word, a.g.cs, a.e, side);
+    for (int k = 0; k < a.sc.nf; ++k) {
+        const float4 ph = ntff_phase(a.sc, n, k);
+        ntff_add<A>(a.ntff + ((long long)k * 12 + (F ? 0 : 6)) * P + p, P, x, F ? ph.z : ph.x, F ? ph.w : ph.y);
+    }
+}
 template <int F>
 __device__ __forceinline__ void res_ntff(const ResArgs& a, unsigned n, unsigned t, unsigned nt) {
-    const long long cs = a.g.cs;
-    const int P = a.n_patches;
-    for (unsigned p = t; p < unsigned(P); p += nt) {
-        const unsigned meta = a.patch[p];
-        const int axis = meta & 3;
+    for (unsigned p = t; p < unsigned(a.n_patches); p += nt) {
+        const unsigned meta = __ldg(a.patch + p);
         const float side = (meta & 4) ? 1.0f : -1.0f;
-        const int u = (axis + 1) % 3, v = (axis + 2) % 3;
-        auto at = [&](int m) { return a.patch[(long long)m * P + p]; };
-        float f[3] = {0, 0, 0}, nrm[3] = {0, 0, 0}, o[3];
-        nrm[axis] = side;
-        if (F == 0) {
-            f[u] = 0.5f * (a.e[u * cs + at(1)] + a.e[u * cs + at(2)]);
-            f[v] = 0.5f * (a.e[v * cs + at(3)] + a.e[v * cs + at(4)]);
-            o[0] = f[1] * nrm[2] - f[2] * nrm[1];
-            o[1] = f[2] * nrm[0] - f[0] * nrm[2];
-            o[2] = f[0] * nrm[1] - f[1] * nrm[0];
-        } else {
-            f[u] = 0.25f * (a.h[u * cs + at(5)] + a.h[u * cs + at(6)] + a.h[u * cs + at(7)] + a.h[u * cs + at(8)]);
-            f[v] = 0.25f * (a.h[v * cs + at(9)] + a.h[v * cs + at(10)] + a.h[v * cs + at(11)] + a.h[v * cs + at(12)]);
-            o[0] = nrm[1] * f[2] - nrm[2] * f[1];
-            o[1] = nrm[2] * f[0] - nrm[0] * f[2];
-            o[2] = nrm[0] * f[1] - nrm[1] * f[0];
-        }
-        for (int k = 0; k < a.sc.nf; ++k) {
-            const float4 ph = res_phase(a.sc, a.sc.far, n, k, true);
-            const float p0 = F ? ph.z : ph.x, p1 = F ? ph.w : ph.y;
-            float* acc = a.ntff + ((long long)k * 12 + (F ? 0 : 6)) * P + p;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                acc[(long long)(2 * c) * P] += p0 * o[c];
-                acc[(long long)(2 * c + 1) * P] += p1 * o[c];
-            }
-        }
+        if ((meta & 3) == 0) res_ntff_patch<F, 0>(a, n, p, side);
+        else if ((meta & 3) == 1) res_ntff_patch<F, 1>(a, n, p, side);
+        else res_ntff_patch<F, 2>(a, n, p, side);
     }
 }
 
