@@ -249,10 +249,9 @@ __device__ __forceinline__ void adj_half(const AdjResArgs& A, const AdjNode* X, 
                                          unsigned first, long long n) {
     const ResArgs& a = A.r;
     const float2 z = make_float2(a.neg0, a.neg0);
-    unsigned row = a.quads(first), col = first - row * a.quads.d;
-    unsigned i = a.rows(row), j = row - i * a.rows.d;
-    while (i < unsigned(a.g.n0)) {
-        const AdjPos p{row, row * unsigned(a.g.p2) + col * 4u, int(i), int(j), int(col * 4u)};
+    ResWalk<F == 0> at(a, first);   // the second phase walks backwards (res_half)
+    while (at.inside(a)) {
+        const AdjPos p{unsigned(at.row), unsigned(at.row) * unsigned(a.g.p2) + unsigned(at.col) * 4u, at.i, at.j, at.col * 4};
         const unsigned ido = unsigned(C) * unsigned(a.g.cs) + p.id;
         const int nk = a.g.n2 - p.k;
         if constexpr (F) {
@@ -288,12 +287,7 @@ __device__ __forceinline__ void adj_half(const AdjResArgs& A, const AdjNode* X, 
             v.b = f2::pick(nk > 2, nk > 3, v.b, make_float2(0.f, 0.f));
             st4(a.e + ido, v);
         }
-        col += a.dq;
-        row += a.drow;
-        j += a.dj;
-        i += a.di;
-        if (col >= a.quads.d) { col -= a.quads.d; ++row; ++j; }
-        if (j >= a.rows.d) { j -= a.rows.d; ++i; }
+        at.next(a);
     }
 }
 

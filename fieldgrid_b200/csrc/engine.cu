@@ -796,6 +796,7 @@ void resident_shape(const Session& s, ResArgs& a) {
     const unsigned q = unsigned(g.n2 + 3) / 4, pass = unsigned(s.res_blocks) * unsigned(s.res_groups);
     a.quads = FastDiv(q);
     a.rows = FastDiv(unsigned(g.n1));
+    a.last_row = unsigned(g.n0) * unsigned(g.n1) - 1u;
     a.drow = pass / q;
     a.dq = pass % q;
     a.di = a.drow / unsigned(g.n1);
