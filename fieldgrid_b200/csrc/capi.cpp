@@ -11,6 +11,8 @@
 #include <string>
 #include <vector>
 
+#include <sys/mman.h>
+
 #include "../../include/fieldgrid.h"
 #include "engine.hpp"
 
@@ -84,10 +86,40 @@ struct fg_gpu { Gpu* g; };
 struct fg_sim { HostSim* s; };
 struct fg_session { Session* s; };
 struct fg_far { Far f; };
+// A record's array: not cleared (the read-back fills it), on huge pages where the system grants them
+// (the first faults of a large read-back cost as much as its copy).
+struct HostArray {
+    float* p = nullptr;
+    size_t n = 0;
+    bool resize(size_t len) {   // false: no memory
+        std::free(p);
+        n = len;
+        p = nullptr;
+        if (!len) return true;
+        const size_t huge = size_t(2) << 20, bytes = len * 4;
+        if (bytes < 2 * huge) {
+            p = static_cast<float*>(std::malloc(bytes));
+        } else {
+            p = static_cast<float*>(std::aligned_alloc(huge, (bytes + huge - 1) & ~(huge - 1)));
+            if (p) madvise(p, bytes, MADV_HUGEPAGE);
+        }
+        if (!p) n = 0;
+        return p != nullptr;
+    }
+    float* data() { return p; }
+    const float* data() const { return p; }
+    size_t size() const { return n; }
+    bool empty() const { return n == 0; }
+    HostArray() = default;
+    HostArray(const HostArray&) = delete;
+    HostArray& operator=(const HostArray&) = delete;
+    ~HostArray() { std::free(p); }
+};
+
 struct fg_record {
     uint64_t steps = 0, ports = 0;
     double decay_db = 0;
-    std::vector<float> series, plane, ntff, e, h;
+    HostArray series, plane, ntff, e, h;
     bool has_fields = false;
     uint64_t h2d = 0, d2h = 0;
 };
@@ -298,19 +330,19 @@ int fg_run(fg_gpu* g, const fg_sim* sim, uint64_t driven, const fg_pulse* pulse,
     rec->steps = steps;
     rec->ports = session_ports(s);
     rec->decay_db = decay;
-    rec->series.resize(std::min<uint64_t>(steps, extras->max_steps) * rec->ports * 2);
+    const char* full = "out of host memory for the record";
+    if (!rec->series.resize(std::min<uint64_t>(steps, extras->max_steps) * rec->ports * 2)) return fail(FG_ERR_TOO_LARGE, full, err, errlen);
     rc = session_read(s, "series", rec->series.data(), rec->series.size(), e);
     if (!rc) {
-        rec->plane.resize(session_plane_len(s));
+        if (!rec->plane.resize(session_plane_len(s))) return fail(FG_ERR_TOO_LARGE, full, err, errlen);
         rc = session_read(s, "plane", rec->plane.data(), rec->plane.size(), e);
     }
     if (!rc) {
-        rec->ntff.resize(session_ntff_len(s));
+        if (!rec->ntff.resize(session_ntff_len(s))) return fail(FG_ERR_TOO_LARGE, full, err, errlen);
         rc = session_read(s, "ntff", rec->ntff.data(), rec->ntff.size(), e);
     }
     if (!rc && extras->keep_fields) {
-        rec->e.resize(3 * sim->s->nn);
-        rec->h.resize(3 * sim->s->nn);
+        if (!rec->e.resize(3 * sim->s->nn) || !rec->h.resize(3 * sim->s->nn)) return fail(FG_ERR_TOO_LARGE, full, err, errlen);
         rc = session_read(s, "e", rec->e.data(), rec->e.size(), e);
         if (!rc) rc = session_read(s, "h", rec->h.data(), rec->h.size(), e);
         rec->has_fields = true;
@@ -329,7 +361,7 @@ uint64_t fg_record_steps(const fg_record* r) { return r ? r->steps : 0; }
 uint64_t fg_record_ports(const fg_record* r) { return r ? r->ports : 0; }
 double fg_record_decay_db(const fg_record* r) { return r ? r->decay_db : 0.0; }
 
-static const float* view(const std::vector<float>& v, uint64_t* len) {
+static const float* view(const HostArray& v, uint64_t* len) {
     if (len) *len = v.size();
     return v.empty() ? nullptr : v.data();
 }

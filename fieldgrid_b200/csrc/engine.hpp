@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -44,6 +45,7 @@ struct Gpu {
     // through the two buffers in turn, so filling one overlaps the transfer of the other
     void* stage[2] = {nullptr, nullptr};
     void* stage_ev[2] = {nullptr, nullptr};   // cudaEvent_t: the last transfer out of each buffer
+    std::mutex stage_lock;                    // one upload or read-back through the buffers at a time
     // the arena of the last session freed on this device, kept for the next session of a similar
     // size (runs of one grid after another skip the allocation and its release)
     void* spare = nullptr;
