@@ -211,6 +211,12 @@ __global__ void k_far_finish(const double* __restrict__ partial, int parts, int 
     far_finish(s, d, kw, out + 6 * (long long)q);
 }
 
+// Each patch's currents times its area.
+__global__ void k_far_areas(double* __restrict__ jm, const double* __restrict__ area, long long count) {
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < 12 * count; q += (long long)gridDim.x * blockDim.x)
+        jm[q] *= area[q / 12];
+}
+
 // The patches as lines with shared sequences.
 struct Line {
     int first, len, axis, seq;   // seq: offset into the sequence values
@@ -295,12 +301,16 @@ int far_layout(Gpu* g, const double* pos, const double* area, const double* jm, 
         find_lines(pos, int(count), lines, seqs);
         D.lined = lines.size() * 8 <= count;
     }
-    std::vector<double> w(12 * count);
-#pragma omp parallel for schedule(static)
-    for (long long i = 0; i < (long long)count; ++i)
-        for (int x = 0; x < 12; ++x) w[size_t(12 * i + x)] = jm[12 * i + x] * area[i];
-    if (!check(cudaMalloc(&D.jm, std::max<size_t>(w.size(), 1) * 8), "cudaMalloc")) return FG_ERR_CUDA;
-    if (!check(cudaMemcpy(D.jm, w.data(), w.size() * 8, cudaMemcpyHostToDevice), "cudaMemcpy")) return FG_ERR_CUDA;
+    // the currents, then their areas behind them for the products
+    if (!check(cudaMalloc(&D.jm, std::max<size_t>(13 * count, 1) * 8), "cudaMalloc")) return FG_ERR_CUDA;
+    if (count) {
+        double* a = D.jm + 12 * count;
+        if (!check(cudaError_t(staged_upload(g, D.jm, jm, 12 * count * 8, nullptr)), "cudaMemcpy") ||
+            !check(cudaError_t(staged_upload(g, a, area, count * 8, nullptr)), "cudaMemcpy"))
+            return FG_ERR_CUDA;
+        k_far_areas<<<148 * 8, 256>>>(D.jm, a, (long long)count);
+        if (!check(cudaGetLastError(), "k_far_areas")) return FG_ERR_CUDA;
+    }
     if (D.lined) {
         // lines of one sequence, in their order, four to a group
         std::stable_sort(lines.begin(), lines.end(), [](const Line& a, const Line& b) { return a.seq < b.seq; });
