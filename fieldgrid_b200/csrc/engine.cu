@@ -504,9 +504,13 @@ CleanPlan plan_clean(const HostSim& sim, const Geom& g, bool z_layer, int seg_fi
     const int jfirst = anchor < 0 ? out.lo[1] : anchor - TMA_TJ * ((anchor - out.lo[1] + TMA_TJ - 1) / TMA_TJ);
     const int jt = (out.hi[1] - jfirst + TMA_TJ - 1) / TMA_TJ;
     const int xw = out.hi[0] - out.lo[0];
-    // x-planes per block: enough blocks for several waves of 3 blocks per SM, at most TMA_SEGMAX
+    // x-planes per block: at least two waves of two blocks per SM, at most TMA_SEGMAX planes. A block pays
+    // for its tables, its pipeline's start and a plane recomputed; nine waves of 8-plane blocks cost more
+    // than a ragged second wave (a step at 257x257x193: 315 us with 8 planes, 292 with 17, 282 with 29 or
+    // 39, 302 with 58; 201^3: 226 with 8, 199 with 30, 219 with 60; 301x281x321: 450 with 16, 426 with 47
+    // or 56)
     int seg = TMA_SEGMAX;
-    while (seg > 8 && (long long)kt * jt * ((xw + seg - 1) / seg) < 148 * 3 * 6) seg /= 2;
+    while (seg > 8 && (long long)kt * jt * ((xw + seg - 1) / seg) < 148 * 2 * 2) seg /= 2;
     if (seg_fixed > 0) seg = std::min(seg_fixed, TMA_SEGMAX);
     std::vector<int2> sg = segs;
     if (sg.empty()) {
