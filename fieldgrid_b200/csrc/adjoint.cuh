@@ -190,7 +190,7 @@ struct FluxJob {
     // design edges, 640 steps: 142 MB against 10 checkpoints of 78 MB; the re-runs were half the
     // backward's device time).
     bool keep_history() const {
-        const size_t p2 = (sim->n[2] + 31) & ~size_t(31), cs = (sim->n[0] * sim->n[1] * p2 + 31) & ~size_t(31);
+        const size_t p2 = (sim->n[2] + 15) & ~size_t(15), cs = (sim->n[0] * sim->n[1] * p2 + 31) & ~size_t(31);
         const size_t per = 2 * 3 * cs * 4 + sim->debye_edges.size() * sim->poles.size() * 4;   // without its psi
         return uint64_t(N) * info.size() * 8 <= per * S + 2 * L * info.size() * 8;
     }
@@ -567,7 +567,7 @@ struct FluxJob {
         if ((rc = event(&e0, true)) || (rc = event(&e1, true))) return rc;
         FG_CUDA(cudaEventRecord(e0, st));
         for (uint64_t left = N; left > 0;) {
-            A.r.steps = int(std::min<uint64_t>(left, RES_MAX_STEPS));
+            A.r.steps = int(std::min<uint64_t>(left, resident_steps(*s)));
             A.n_hi = (long long)left;
             rc = with_adj_resident(s->cid_bytes, s->res_cluster, [&](auto kern) -> int {
                 return launch_res(*s, kern, A, adj_res_smem(g), st, err);

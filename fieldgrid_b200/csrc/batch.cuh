@@ -191,7 +191,7 @@ int batch_plan_resident(Batch& B, int share, std::string& err) {
     return FG_OK;
 }
 
-// `k` steps (at most RES_MAX_STEPS) of every grid as resident launches on the grids' streams, between the
+// `k` steps (at most resident_steps) of every grid as resident launches on the grids' streams, between the
 // batch stream's earlier and later work. The launches go to `share` streams in turn.
 int batch_resident(Batch& B, uint64_t k, std::string& err) {
     FG_CUDA(cudaEventRecord(B.fork, B.stream));
@@ -524,7 +524,8 @@ int batch_step(Batch& B, uint64_t k, std::string& err) {
     while (done < k) {
         const int parity = int(B.steps & 1);
         if (B.share > 0 && k - done >= BATCH_RESIDENT_STEPS) {
-            const uint64_t m = std::min<uint64_t>(k - done, RES_MAX_STEPS);
+            uint64_t m = k - done;
+            for (Session* s : B.s) m = std::min(m, resident_steps(*s));
             const int rc = batch_resident(B, m, err);
             if (rc) return rc;
             done += m;

@@ -133,12 +133,15 @@ int staged_upload(Gpu* g, void* dst, const void* src, size_t bytes, void* stream
     return staged_fill(g, dst, bytes, st, [s8](char* buf, size_t off, size_t n) { std::memcpy(buf, s8 + off, n); });
 }
 
-// Steps of one resident launch at most (a bound on the time one kernel holds the GPU).
+// Steps of one resident launch at most, and nodes times steps (a bound on the time one kernel holds the GPU).
 constexpr uint64_t RES_MAX_STEPS = 1024;
-// Nodes of a grid stepped resident at most: beyond, the fields and psi (24 to 35 B per node) leave the
-// L2. Measured per step against the TMA march's graphs and the separate kernels': 65^3 10.0 us against
-// 35.1 and 21.1; 121^3 with Debye spheres 31 against 64 and 57; 160^3 85 against 110 and 161.
-constexpr long long RES_MAX_NODES = 4 << 20;
+constexpr long long RES_MAX_WORK = 1LL << 32;
+// Nodes of a grid stepped resident at most. In the fused mode the TMA march's graphs take over where they
+// move fewer bytes at the HBM rate; the separate kernels are slower at every size (32-bit field offsets
+// bound it). Measured us per step, resident / march / separate: 65^3 9 / 35 / 21; 121^3 with Debye
+// spheres 30 / 64 / 57; 145^3 56 / 97 / 130; 201^3 129 / 175 / 320; 261^3 265 / 335 / 668;
+// 299^3 490 / 465.
+constexpr long long RES_MAX_FUSED = 22LL << 20, RES_MAX_SEPARATE = 1LL << 28;
 // 4-node groups of a grid stepped by one cluster at most: its barrier is shorter than a grid-wide one,
 // but 16 SMs share the work (29x19x14: 4.1 us a step against 5.2; 25^3: 6.5 against 6.5).
 constexpr long long RES_CLUSTER_GROUPS = 4096;
@@ -341,8 +344,7 @@ struct Session {
     cudaEvent_t shell_fork = nullptr, shell_join = nullptr;
     int prio_lo = 0, prio_hi = 0;
     bool capturing = false;
-    // whole calls of session_step as one resident launch (stencil_resident.cuh), where the grid's
-    // state stays in L2
+    // whole calls of session_step as resident launches (stencil_resident.cuh)
     bool resident = false;
     int res_blocks = 0, res_groups = 0;
     bool res_cluster = false;
@@ -828,7 +830,9 @@ int plan_resident(Session& s, int share, std::string& err) {
     if (!coop) return FG_OK;
     const long long total = (long long)g.n0 * g.n1 * ((g.n2 + 3) / 4);
     auto groups_of = [&](long long blocks) {   // per block and pass, in whole warps
-        return int(std::min<long long>(RES_GROUPS / share / 32 * 32, std::max<long long>(32, ((total + blocks - 1) / blocks + 31) / 32 * 32)));
+        const long long most = RES_GROUPS / share / 32 * 32, passes = std::max<long long>(1, (total + blocks * most - 1) / (blocks * most));
+        const long long even = ((total + blocks * passes - 1) / (blocks * passes) + 31) / 32 * 32;   // passes of one size
+        return int(std::min(most, std::max<long long>(32, passes <= 4 ? even : most)));
     };
     s.res_cluster = total <= RES_CLUSTER_GROUPS;
     const int most = s.res_cluster ? RES_CLUSTER : sms;
@@ -846,6 +850,11 @@ int plan_resident(Session& s, int share, std::string& err) {
     if (per < 1) return FG_OK;
     s.resident = true;
     return FG_OK;
+}
+
+// Steps of one launch for a session.
+uint64_t resident_steps(const Session& s) {
+    return std::min<uint64_t>(RES_MAX_STEPS, std::max<uint64_t>(16, uint64_t(RES_MAX_WORK / s.geom.nn)));
 }
 
 // The launch shape and index arithmetic shared by the resident kernels of a session.
@@ -1539,7 +1548,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     g.n0 = int(n0); g.n1 = int(n1); g.n2 = int(n2);
     g.pml = int(sim.pml);
     g.nn = (long long)nn;
-    g.p2 = int((n2 + 31) & ~size_t(31));
+    g.p2 = int((n2 + 15) & ~size_t(15));
     const size_t nnp = n0 * n1 * size_t(g.p2);   // device nodes, rows padded to the pitch
     g.cs = (long long)((nnp + 31) & ~size_t(31));
     const long long cs = g.cs;
@@ -1552,10 +1561,10 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     // adjacent, each slab 128-byte aligned, z-slab rows padded to pw slots
     g.pw = int((2 * sim.pml + 3) & ~size_t(3));
     g.pk = int((n2 + 3) & ~size_t(3));
-    // the k axis as the device keeps it: on grids small enough to step resident, with its layer's slots
+    // the k axis as the device keeps it: on grids of a size that steps resident, with its layer's slots
     // numbered by 4-node groups where that is possible
     std::vector<AxisNode> kax_node = sim.ax[2].node;
-    s->k_quads = (long long)nn <= RES_MAX_NODES && n0 + n1 + n2 <= size_t(RES_MAX_AXES) && res_k_slots(kax_node, sim.pml, g.pw);
+    s->k_quads = (long long)nn <= (s->fused ? RES_MAX_FUSED : RES_MAX_SEPARATE) && 3 * g.cs < (1LL << 32) && n0 + n1 + n2 <= size_t(RES_MAX_AXES) && res_k_slots(kax_node, sim.pml, g.pw);
     long long psi_total = 0, psi_hbase = 0;
     for (int e = 0; e < 2; ++e) {
         if (e == 1) psi_hbase = psi_total;
@@ -2323,7 +2332,7 @@ int session_step(Session* s, uint64_t k, std::string& err) {
     uint64_t done = 0;
     if (s->resident) {
         while (done < k) {
-            const uint64_t m = std::min<uint64_t>(k - done, RES_MAX_STEPS);
+            const uint64_t m = std::min<uint64_t>(k - done, resident_steps(*s));
             const int rc = launch_resident(*s, m, err);
             if (rc) return rc;
             done += m;

@@ -12,7 +12,7 @@
 namespace fg {
 
 // Node geometry shared by every kernel. On the device a row of n2 nodes is stored with pitch p2
-// (n2 rounded up to 32, so rows start 128-byte aligned and TMA strides are legal): the device
+// (n2 rounded up to 16: TMA strides and 4-node loads are legal, a row of class ids is whole 16-byte units): the device
 // node index is (i*n1 + j)*p2 + k. Fields are component-major with component stride cs
 // (>= n0*n1*p2). The psi slabs follow the reference's layout (sim.rs:659-665), except that a
 // z slab (derivative along k) pads its rows of 2 pml slots to pw and the x and y slabs theirs of n2

@@ -21,6 +21,7 @@
 // to the other buffer set, so that the latest set stays the one the parity of the step count names.
 #pragma once
 
+#include <type_traits>
 #include <vector>
 
 #include "kernels.cuh"
@@ -223,19 +224,16 @@ __device__ __forceinline__ void q_psi(Quad& t, Quad& psi, const Quad& d, const Q
     t = t + psi;
 }
 
-// The class ids of 4 nodes in one load.
+// The class ids of 4 nodes, as loaded and one by one.
 template <typename CID>
-__device__ __forceinline__ uint4 res_ids(const CID* p) {
-    if constexpr (sizeof(CID) == 1) {
-        const unsigned v = __ldg(reinterpret_cast<const unsigned*>(p));
-        return make_uint4(v & 255u, v >> 8 & 255u, v >> 16 & 255u, v >> 24);
-    } else if constexpr (sizeof(CID) == 2) {
-        const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
-        return make_uint4(v.x & 65535u, v.x >> 16, v.y & 65535u, v.y >> 16);
-    } else {
-        return __ldg(reinterpret_cast<const uint4*>(p));
-    }
-}
+using IdWords = std::conditional_t<sizeof(CID) == 1, unsigned, std::conditional_t<sizeof(CID) == 2, uint2, uint4>>;
+template <typename CID>
+__device__ __forceinline__ IdWords<CID> res_load_ids(const CID* p) { return __ldg(reinterpret_cast<const IdWords<CID>*>(p)); }
+__device__ __forceinline__ uint4 res_each(unsigned v) { return make_uint4(v & 255u, v >> 8 & 255u, v >> 16 & 255u, v >> 24); }
+__device__ __forceinline__ uint4 res_each(uint2 v) { return make_uint4(v.x & 65535u, v.x >> 16, v.y & 65535u, v.y >> 16); }
+__device__ __forceinline__ uint4 res_each(uint4 v) { return v; }
+template <typename CID>
+__device__ __forceinline__ uint4 res_ids(const CID* p) { return res_each(res_load_ids(p)); }
 
 // One component C of the field (F = 1: E from H, F = 0: H from E) on the 4 nodes from (i, j, k)
 // (cpu.rs:48-167): its two curl terms R - S, R the difference along i or j that its row decides (x: j,
@@ -247,8 +245,8 @@ __device__ __forceinline__ uint4 res_ids(const CID* p) {
 // reference's does by the cleared factors. Every field load comes before the first store.
 template <int C, int F, typename CID>
 __device__ __forceinline__ void res_update(const ResArgs& a, const ResNode* X, const ResNode* Y, const float* Z, int np2, unsigned row,
-                                           int i, int j, int k, const float* src, const float* own, float* out,
-                                           const float* psi_in, float* psi_out) {
+                                           int i, int j, int k, IdWords<CID> words, const float* src, const float* own,
+                                           float* out, const float* psi_in, float* psi_out) {
     const Geom& g = a.g;
     const unsigned id = row * unsigned(g.p2) + unsigned(k), cs = unsigned(g.cs);
     const float2 z = make_float2(a.neg0, a.neg0);
@@ -269,11 +267,23 @@ __device__ __forceinline__ void res_update(const ResArgs& a, const ResNode* X, c
     if constexpr (S_J) s1 = ld4(src + (F ? ids - sj : ids + sj));
     else if constexpr (F) s1 = q_down(s0, k > 0 ? src[ids - 1] : 0.f);
     else s1 = q_up(s0, nk > 4 ? src[ids + 4] : 0.f);
+    // the psi of both differences with the fields: nearly every warp has lanes in the layer along k, and
+    // a load behind the differences would cost it another round of latency
     const ResNode* tr = ALONG_I ? X + i : Y + j;
     const ResHalf fr = tr->f[F];
+    const int sls = S_J ? Y[j].f[F].slot : reinterpret_cast<const int*>(Z + 8 * np2)[k >> 2];
+    const unsigned orr = unsigned(g.psi_off[(F ? 0 : 9) + C * 3 + (ALONG_I ? 0 : 1)]) + unsigned(k) +
+                         (ALONG_I ? unsigned(fr.slot) * unsigned(g.n1) + unsigned(j)
+                                  : unsigned(i) * unsigned(2 * g.pml) + unsigned(fr.slot)) * unsigned(g.pk);
+    const unsigned os = S_J ? unsigned(g.psi_off[(F ? 0 : 9) + C * 3 + 1]) + unsigned(k) +
+                                  (unsigned(i) * unsigned(2 * g.pml) + unsigned(sls)) * unsigned(g.pk)
+                            : unsigned(g.psi_off[(F ? 0 : 9) + C * 3 + 2]) + row * unsigned(g.pw) + unsigned(sls);
+    Quad pr = q_zero(), ps = q_zero();
+    if (fr.slot >= 0) pr = ld4(psi_in + orr);
+    if (sls >= 0) ps = ld4(psi_in + os);
     float2 ca0, ca1, cb0, cb1;
     if constexpr (F) {
-        const uint4 cid = res_ids(static_cast<const CID*>(a.node_class) + id);
+        const uint4 cid = res_each(words);
         const float* t = reinterpret_cast<const float*>(a.classes) + C;
         const float fa = __ldg(t + cid.x * 8), fb = __ldg(t + cid.x * 8 + 4);   // most groups hold one class
         ca0 = ca1 = make_float2(fa, fa);
@@ -287,33 +297,19 @@ __device__ __forceinline__ void res_update(const ResArgs& a, const ResNode* X, c
     const Quad dr = F ? r0 - r1 : r1 - r0, ds = F ? s0 - s1 : s1 - s0;
     Quad R = q_mul(dr, q_bc(fr.inv), z), S;
     if (fr.slot >= 0) {
-        const unsigned o = unsigned(g.psi_off[(F ? 0 : 9) + C * 3 + (ALONG_I ? 0 : 1)]) + unsigned(k) +
-                           (ALONG_I ? unsigned(fr.slot) * unsigned(g.n1) + unsigned(j)
-                                    : unsigned(i) * unsigned(2 * g.pml) + unsigned(fr.slot)) * unsigned(g.pk);
-        Quad p = ld4(psi_in + o);
-        q_psi(R, p, dr, q_bc(fr.b), q_bc(tr->c[F]), q_bc(fr.raw), z);
-        st4(psi_out + o, p);
+        q_psi(R, pr, dr, q_bc(fr.b), q_bc(tr->c[F]), q_bc(fr.raw), z);
+        st4(psi_out + orr, pr);
     }
     if constexpr (S_J) {
         const ResHalf fs = Y[j].f[F];
         S = q_mul(ds, q_bc(fs.inv), z);
-        if (fs.slot >= 0) {
-            const unsigned o = unsigned(g.psi_off[(F ? 0 : 9) + C * 3 + 1]) + unsigned(k) +
-                               (unsigned(i) * unsigned(2 * g.pml) + unsigned(fs.slot)) * unsigned(g.pk);
-            Quad p = ld4(psi_in + o);
-            q_psi(S, p, ds, q_bc(fs.b), q_bc(Y[j].c[F]), q_bc(fs.raw), z);
-            st4(psi_out + o, p);
-        }
+        if (sls >= 0) q_psi(S, ps, ds, q_bc(fs.b), q_bc(Y[j].c[F]), q_bc(fs.raw), z);
     } else {
         S = q_mul(ds, ld4(Z + (F ? 1 : 0) * np2 + k), z);
-        const int sl = reinterpret_cast<const int*>(Z + 8 * np2)[k >> 2];
-        if (sl >= 0) {
-            const unsigned o = unsigned(g.psi_off[(F ? 0 : 9) + C * 3 + 2]) + row * unsigned(g.pw) + unsigned(sl);
-            Quad p = ld4(psi_in + o);
-            q_psi(S, p, ds, ld4(Z + (F ? 4 : 6) * np2 + k), ld4(Z + (F ? 5 : 7) * np2 + k), ld4(Z + (F ? 3 : 2) * np2 + k), z);
-            st4(psi_out + o, p);
-        }
+        if (sls >= 0)
+            q_psi(S, ps, ds, ld4(Z + (F ? 4 : 6) * np2 + k), ld4(Z + (F ? 5 : 7) * np2 + k), ld4(Z + (F ? 3 : 2) * np2 + k), z);
     }
+    if (sls >= 0) st4(psi_out + os, ps);
     const Quad t = C == 1 ? S - R : R - S;
     Quad n;
     if constexpr (F) {
@@ -377,9 +373,19 @@ template <int C, int F, typename CID>
 __device__ __forceinline__ void res_half(const ResArgs& a, const ResNode* X, const ResNode* Y, const float* Z, int np2, unsigned first,
                                          const float* src, const float* own, float* out, const float* psi_in, float* psi_out) {
     ResWalk<F != 0> at(a, first);
+    // the E half's class ids a group ahead: its coefficients' addresses stand when its other loads start
+    const CID* cls = static_cast<const CID*>(a.node_class);
+    auto ids = [&](const ResWalk<F != 0>& w) { return res_load_ids(cls + (unsigned(w.row) * unsigned(a.g.p2) + unsigned(w.col) * 4u)); };
+    IdWords<CID> words{};
+    if (F && at.inside(a)) words = ids(at);
     while (at.inside(a)) {
-        res_update<C, F, CID>(a, X, Y, Z, np2, unsigned(at.row), at.i, at.j, at.col * 4, src, own, out, psi_in, psi_out);
-        at.next(a);
+        ResWalk<F != 0> nx = at;
+        nx.next(a);
+        IdWords<CID> ahead{};
+        if (F && nx.inside(a)) ahead = ids(nx);
+        res_update<C, F, CID>(a, X, Y, Z, np2, unsigned(at.row), at.i, at.j, at.col * 4, words, src, own, out, psi_in, psi_out);
+        at = nx;
+        words = ahead;
     }
 }
 
