@@ -344,6 +344,7 @@ struct FluxJob {
             FG_CUDA(cudaMemcpyAsync(c.e, s->e, fbytes, cudaMemcpyDeviceToDevice, st));
             FG_CUDA(cudaMemcpyAsync(c.h, s->h, fbytes, cudaMemcpyDeviceToDevice, st));
             FG_CUDA(cudaMemcpyAsync(c.psi, s->psi, pbytes, cudaMemcpyDeviceToDevice, st));
+            if ((rc = debye_states(*s, false, st, err))) return rc;
             if (nd_s) FG_CUDA(cudaMemcpyAsync(c.deb, s->debye_state, nd_s * 4, cudaMemcpyDeviceToDevice, st));
             if ((rc = session_step(s, std::min<uint64_t>(L, N - q * L), err))) return rc;
         }
@@ -454,6 +455,7 @@ struct FluxJob {
             FG_CUDA(cudaMemcpyAsync(s->h, cks[q].h, fbytes, cudaMemcpyDeviceToDevice, st));
             FG_CUDA(cudaMemcpyAsync(s->psi, cks[q].psi, pbytes, cudaMemcpyDeviceToDevice, st));
             if (nd_s) FG_CUDA(cudaMemcpyAsync(s->debye_state, cks[q].deb, nd_s * 4, cudaMemcpyDeviceToDevice, st));
+            s->rd_dense = false;   // the re-run steps on the list
             s->steps = a;
             // the step counter at a, the history slots of ring half q & 1
             if ((r = set_base((long long)(a - (q & 1) * L), true, unsigned(a)))) return r;

@@ -314,17 +314,18 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_adj_resident(const __grid_co
     const int w = threadIdx.x >> 5, comp = w % 3;
     const unsigned groups = blockDim.x / 3u, G = gridDim.x, b = blockIdx.x;
     const unsigned first = b * groups + unsigned(w / 3) * 32u + (threadIdx.x & 31u);
-    const int t = int((unsigned(w) * G + b) * 32u + (threadIdx.x & 31u)), nt = int(G * blockDim.x);
-    const int poles = a.n_debye ? int(a.debye_table[0]) : 0;
+    auto t = [] { return int(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32u + (threadIdx.x & 31u)); };   // k_resident's
+    auto nt = [] { return int(gridDim.x * blockDim.x); };
     unsigned target = 0;
     for (long long n = A.n_hi - 1; n >= A.n_hi - a.steps; --n) {
         if (a.n_debye) {
-            for (int q = t; q < a.n_debye; q += nt) {
+            for (int q = t(); q < a.n_debye; q += nt()) {
                 const long long fi = a.debye_f[q];
                 float l = a.e[fi] + A.lold[q];
                 const int dw = A.dwin[q];
                 if (dw >= 0) l += adj_source<1>(A, n, dw & 1, dw >> 1);
                 const float wd = a.debye_dd[q], cb = a.debye_cb[q];
+                const int poles = int(a.debye_table[0]);
                 float d = 0.0f;
                 for (int k = 0; k < poles; ++k) d += wd * a.debye_table[2 + 2 * k] * A.ls[(long long)k * a.n_debye + q];
                 const float le = l + d;
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_adj_resident(const __grid_co
             if (!res_barrier<CLUSTER>(a, target += G)) return;
         }
         const long long slot = n * a.n_design;
-        for (int q = t; q < a.n_design; q += nt) {   // adj_grad; no design edge is a Debye edge
+        for (int q = t(); q < a.n_design; q += nt()) {   // adj_grad; no design edge is a Debye edge
             const int4 d = a.design[q];
             const double l = a.e[d.x * g.cs + ((long long)d.y * g.n1 + d.z) * g.p2 + d.w];
             A.ga[q] += l * double(A.hist_e[slot + q]);

@@ -533,6 +533,8 @@ int batch_step(Batch& B, uint64_t k, std::string& err) {
             for (Session* s : B.s) s->steps = B.steps;
             continue;
         }
+        for (Session* s : B.s)   // the graphs step on the Debye lists
+            if (const int rc = debye_states(*s, false, B.stream, err)) return rc;
         if (parity == 0 && k - done >= uint64_t(B.graph_steps) && B.graph_many) {
             FG_CUDA(cudaGraphLaunch(B.graph_many, B.stream));
             done += B.graph_steps;

@@ -350,6 +350,13 @@ struct Session {
     bool res_cluster = false;
     bool k_quads = false;           // a grid of that size, its k slots numbered by 4-node groups
     unsigned* res_bar = nullptr;    // the grid barrier's arrivals
+    // the Debye edges by 4-node groups (resident steps); rd_dense: the pole states are there, not in
+    // debye_state
+    int *rd_index = nullptr, *rd_sums = nullptr;
+    float *rd_dd = nullptr, *rd_state = nullptr;
+    void* rd_tmp = nullptr;
+    size_t rd_tmp_bytes = 0, rd_places = 0;
+    bool rd_built = false, rd_dense = false;
     std::map<int, cudaGraphExec_t> slot_graphs;      // captured steps by (kind, phase t mod 6)
     std::vector<void*> extra_allocs;
 };
@@ -796,10 +803,44 @@ int enqueue_step(Session& s, int parity, std::string& err) {
 // ---- resident stepping ----------------------------------------------------------------------
 
 template <typename F>
-int with_resident(int cid_bytes, bool cluster, F&& f) {
-    if (cid_bytes == 1) return cluster ? f(k_resident<uint8_t, true>) : f(k_resident<uint8_t, false>);
-    if (cid_bytes == 2) return cluster ? f(k_resident<uint16_t, true>) : f(k_resident<uint16_t, false>);
-    return cluster ? f(k_resident<uint32_t, true>) : f(k_resident<uint32_t, false>);
+int with_resident(const Session& s, F&& f) {
+    auto go = [&](auto cid) {
+        using C = decltype(cid);
+        if (s.n_debye) return s.res_cluster ? f(k_resident<C, true, true>) : f(k_resident<C, false, true>);
+        return s.res_cluster ? f(k_resident<C, true, false>) : f(k_resident<C, false, false>);
+    };
+    if (s.cid_bytes == 1) return go(uint8_t{});
+    if (s.cid_bytes == 2) return go(uint16_t{});
+    return go(uint32_t{});
+}
+
+RdMap rd_map(const Session& s) { return RdMap{s.geom, unsigned(s.geom.n2 + 3) / 4, s.debye_f, s.n_debye, s.rd_index}; }
+unsigned rd_blocks(const Session& s) { return unsigned(std::min((s.n_debye + 255) / 256, 148 * 16)); }
+
+// The groups' layout of the Debye edges: places by a scan over the groups that hold one, and the weights.
+int rd_build(Session& s, std::string& err) {
+    if (s.n_debye == 0 || s.rd_built) return FG_OK;
+    const RdMap m = rd_map(s);
+    const unsigned groups = unsigned(s.geom.n0) * unsigned(s.geom.n1) * m.quads;
+    k_rd_mark<<<rd_blocks(s), 256, 0, s.stream>>>(m);   // the arena is clear
+    FG_CUDA(cub::DeviceScan::ExclusiveSum(s.rd_tmp, s.rd_tmp_bytes, s.rd_index, s.rd_sums, int(groups), s.stream));
+    k_rd_places<<<148 * 8, 256, 0, s.stream>>>(s.rd_index, s.rd_sums, groups);
+    k_rd_weights<<<rd_blocks(s), 256, 0, s.stream>>>(m, s.debye_dd, s.rd_dd);
+    FG_CUDA(cudaGetLastError());
+    FG_CUDA(cudaStreamSynchronize(s.stream));   // a batch steps the grid on another stream
+    s.rd_built = true;
+    return FG_OK;
+}
+
+// The pole states to the groups (dense) or to the list, where the steps that come read them.
+int debye_states(Session& s, bool dense, cudaStream_t st, std::string& err) {
+    if (s.n_debye == 0 || s.rd_dense == dense) return FG_OK;
+    const unsigned pole = unsigned(s.rd_places * 12);
+    if (dense) k_rd_move<true><<<rd_blocks(s), 256, 0, st>>>(rd_map(s), s.n_poles, pole, s.debye_state, s.rd_state);
+    else k_rd_move<false><<<rd_blocks(s), 256, 0, st>>>(rd_map(s), s.n_poles, pole, s.debye_state, s.rd_state);
+    FG_CUDA(cudaGetLastError());
+    s.rd_dense = dense;
+    return FG_OK;
 }
 
 // Whether a session's steps may run resident: not where a pipeline is asked for by name
@@ -823,7 +864,7 @@ int with_adj_resident(int cid_bytes, bool cluster, F&& f) {
 int plan_resident(Session& s, int share, std::string& err) {
     const Geom& g = s.geom;
     s.resident = false;
-    if (!s.k_quads) return FG_OK;
+    if (!s.k_quads || (s.n_debye > 0 && !s.rd_index)) return FG_OK;
     int coop = 0, sms = 0, per = 0;
     FG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s.gpu->device));
     FG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.gpu->device));
@@ -839,7 +880,7 @@ int plan_resident(Session& s, int share, std::string& err) {
     s.res_groups = groups_of(most);
     s.res_blocks = s.res_cluster ? RES_CLUSTER : int(std::min<long long>(sms, (total + s.res_groups - 1) / s.res_groups));
     const size_t smem = res_smem(g);
-    const int rc = with_resident(s.cid_bytes, s.res_cluster, [&](auto kern) -> int {
+    const int rc = with_resident(s, [&](auto kern) -> int {
         FG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      int(size_t(res_pad(RES_MAX_AXES + 9)) * 48)));
         if (s.res_cluster) FG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -848,6 +889,7 @@ int plan_resident(Session& s, int share, std::string& err) {
     });
     if (rc) return rc;
     if (per < 1) return FG_OK;
+    if (const int rb = rd_build(s, err)) return rb;
     s.resident = true;
     return FG_OK;
 }
@@ -924,8 +966,11 @@ int launch_resident(Session& s, uint64_t k, std::string& err, cudaStream_t st = 
     a.psi_e = s.psi;
     a.steps = int(k);
     a.counter = s.counter;
-    a.debye_old = s.debye_old;
-    a.debye_state = s.debye_state;
+    a.rd_index = s.rd_index;
+    a.rd_dd = s.rd_dd;
+    a.rd_state = s.rd_state;
+    a.rd_pole = unsigned(s.rd_places * 12);
+    if (const int rc = debye_states(s, true, st ? st : s.stream, err)) return rc;
     a.src = s.sources;
     a.ind = s.inductors;
     a.probes = s.probes;
@@ -947,7 +992,7 @@ int launch_resident(Session& s, uint64_t k, std::string& err, cudaStream_t st = 
     a.hist_cap = s.hist_cap;
     a.hist_e = s.hist_e;
     a.hist_s = s.hist_s;
-    return with_resident(s.cid_bytes, s.res_cluster, [&](auto kern) -> int {
+    return with_resident(s, [&](auto kern) -> int {
         return launch_res(s, kern, a, res_smem(g), st ? st : s.stream, err);
     });
 }
@@ -1767,6 +1812,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     // does not apply (a region with more classes than a local table)
     const size_t nd = sim.debye_edges.size();
     s->n_debye = int(nd);
+    s->n_poles = int(sim.poles.size());
     // size the arena
     const size_t fields = size_t(3 * cs);
     size_t need = 0;
@@ -1795,6 +1841,14 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     need += carve_size(std::max<size_t>(nd, 1) * 8);
     need += carve_size(std::max<size_t>(nd, 1) * 4) * 3;
     need += carve_size(std::max<size_t>(nd * sim.poles.size(), 1) * 4);
+    // the Debye edges by groups, where the grid may step resident (32-bit offsets)
+    const size_t rgroups = n0 * n1 * ((n2 + 3) / 4);
+    s->rd_places = s->k_quads && nd > 0 && nd < (size_t(1) << 31) ? std::min(nd, rgroups) : 0;
+    if (s->rd_places * 12 * std::max<size_t>(sim.poles.size(), 1) >= (size_t(1) << 32)) s->rd_places = 0;
+    if (s->rd_places) {
+        FG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, s->rd_tmp_bytes, (const int*)nullptr, (int*)nullptr, int(rgroups), nullptr));
+        need += carve_size(rgroups * 4) * 2 + carve_size(s->rd_places * 48) * (1 + sim.poles.size()) + carve_size(s->rd_tmp_bytes);
+    }
     // the host records, set-up only: packed to 8 bytes while staged where the device nodes allow
     const bool pack_debye = nnp < (size_t(1) << 30);
     need += carve_size(std::max<size_t>(nd, 1) * (pack_debye ? sizeof(PackedDebye) : sizeof(DebyeEdge)));
@@ -1867,6 +1921,13 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     s->debye_cb = carve<float>(cur, std::max<size_t>(nd, 1));
     s->debye_old = carve<float>(cur, std::max<size_t>(nd, 1));
     s->debye_state = carve<float>(cur, std::max<size_t>(nd * sim.poles.size(), 1));
+    if (s->rd_places) {
+        s->rd_index = carve<int>(cur, rgroups);
+        s->rd_sums = carve<int>(cur, rgroups);
+        s->rd_dd = carve<float>(cur, s->rd_places * 12);
+        s->rd_state = carve<float>(cur, s->rd_places * 12 * sim.poles.size());
+        s->rd_tmp = carve<char>(cur, s->rd_tmp_bytes);
+    }
     void* debye_raw = carve<char>(cur, std::max<size_t>(nd, 1) * (pack_debye ? sizeof(PackedDebye) : sizeof(DebyeEdge)));
     s->debye_table = carve<float>(cur, debye_table.size());
     float* d_pulse = carve<float>(cur, std::max<size_t>(t_pulse.size(), 1));
@@ -2314,6 +2375,7 @@ int session_reset(Session* s, std::string& err) {
     if (s->n_debye) {
         FG_CUDA(cudaMemsetAsync(s->debye_old, 0, size_t(s->n_debye) * 4, st));
         FG_CUDA(cudaMemsetAsync(s->debye_state, 0, size_t(s->n_debye) * size_t(std::max(s->n_poles, 1)) * 4, st));
+        s->rd_dense = false;   // the next resident step takes the list's
     }
     if (s->fold && s->nfold)
         FG_CUDA(cudaMemsetAsync(s->fstate, 0, size_t(s->nfold) * size_t(std::max(s->n_poles, 1)) * 4, st));
@@ -2510,6 +2572,7 @@ int session_kernel_times(Session* s, uint64_t steps, std::vector<std::pair<std::
     std::vector<int> counts;
     // the two-step mode times double steps (one stream) and reports each kernel's time per step
     const uint64_t per = s->slots ? 2 : 1;
+    if (const int rc = debye_states(*s, false, s->stream, err)) return rc;
     for (uint64_t q = 0; q < steps; q += per) {
         marks.clear();
         if (s->slots) {

@@ -1,7 +1,6 @@
 // Many time steps in one launch, for grids whose state stays in L2: a cooperative kernel with the
 // whole grid's blocks resident steps E and H in place, half a step at a time, with a grid-wide
-// barrier between the halves (two per step; a third where Debye edges or a design history follow the
-// E half).
+// barrier between the halves (two per step; a third where a design history follows the E half).
 //
 // The march kernels move each field once per step through HBM, but a march is a chain of planes: a
 // small grid leaves most SMs idle behind it (65^3: 42 blocks, 33 us a step). In place, a half step
@@ -10,11 +9,18 @@
 // (72 B per node) and two barriers instead of three to six kernel launches.
 //
 // Phase A of step n: new H from E (psi of H included); the records that read E after step n - 1
-// (port voltages, running DFTs of E, the NTFF box's M); each Debye edge's and design edge's E^n.
-// Phase B: new E from H, the source and the inductors on the edges of the block's own nodes; the
+// (port voltages, running DFTs of E, the NTFF box's M); each design edge's E^n.
+// Phase B: new E from H with the Debye ADE, the source and the inductors on the edges of the block's own nodes; the
 // records that read H^n+1/2 (port currents, DFTs of H, the box's J). E does not change in phase A nor
 // H in phase B, so each record reads a settled field without a barrier of its own.
-// Phase C (only with Debye edges or a design history): the Debye ADE and the design edges' curl terms.
+// Phase C (only with a design history): the design edges' curl terms.
+//
+// The Debye ADE needs an edge's E before and after its update, both in the hands of the thread that
+// updates it, so it runs there, on weights and pole states laid out by 4-node groups (dense in the groups
+// that hold a Debye edge, 0 on their other edges, which leaves those as they are). As a pass of its own
+// over the edge list it cost a save of E, a third barrier and 41 bytes an edge: 41^3 9.0 us a step
+// against 6.3 now, 89^3 18.6 against 16.8, 121^3 31.2 against 28.5 (each a fifth of its spheres Debye;
+// 5.8, 14.4 and 26.7 without them).
 //
 // The arithmetic and its order are those of the other pipelines (cpu.rs:48-167, :239-265, :291-415),
 // so the fields equal theirs bit for bit. A launch of an odd number of steps writes its first step
@@ -59,11 +65,14 @@ struct ResArgs {
     FastDiv quads, rows;                      // 4-node groups per row; rows per plane
     unsigned last_row;                        // the grid's last row
     unsigned dq, drow, dj, di;                // a pass of the launch over its groups, as rows and groups; its rows as planes and rows
-    // Debye edges
+    // Debye edges: the list (the adjoint's) and the layout by groups
     const long long* debye_f;
     const float *debye_dd, *debye_cb, *debye_table;
-    float *debye_old, *debye_state;
     int n_debye;
+    const int* rd_index;                      // per group: its place among the groups with Debye edges, or -1
+    const float* rd_dd;                       // weights: [place][component][node]
+    float* rd_state;                          // pole states: [pole][place][component][node]
+    unsigned rd_pole;                         // floats of a pole
     // source, inductors, ports
     const DevSource* src;
     DevInductor* ind;
@@ -243,9 +252,9 @@ __device__ __forceinline__ uint4 res_ids(const CID* p) { return res_each(res_loa
 // A node whose update does not run keeps its value by a select; its psi is advanced all the same where
 // the layer covers it: such a psi is read by no update (its edge never runs), and it stays 0 where the
 // reference's does by the cleared factors. Every field load comes before the first store.
-template <int C, int F, typename CID>
+template <int C, int F, typename CID, bool DEBYE>
 __device__ __forceinline__ void res_update(const ResArgs& a, const ResNode* X, const ResNode* Y, const float* Z, int np2, unsigned row,
-                                           int i, int j, int k, IdWords<CID> words, const float* src, const float* own,
+                                           int i, int j, int k, IdWords<CID> words, int dg, const float* src, const float* own,
                                            float* out, const float* psi_in, float* psi_out) {
     const Geom& g = a.g;
     const unsigned id = row * unsigned(g.p2) + unsigned(k), cs = unsigned(g.cs);
@@ -316,6 +325,20 @@ __device__ __forceinline__ void res_update(const ResArgs& a, const ResNode* X, c
         n = q_mul(Quad{ca0, ca1}, f, z) + q_mul(Quad{cb0, cb1}, t, z);
         n.a = f2::pick(cb0.x != 0.f && (S_J || k > 0), cb0.y != 0.f, n.a, f.a);
         n.b = f2::pick(cb1.x != 0.f, cb1.y != 0.f, n.b, f.b);
+        if (DEBYE && dg >= 0) {   // k_debye_post_cb's arithmetic on the group
+            const unsigned o = unsigned(dg) * 12u + 4u * C;
+            const int poles = int(__ldg(a.debye_table));
+            Quad s0 = q_zero();
+            for (int m = 0; m < poles; ++m)
+                s0 = s0 + q_mul(q_bc(0.5f * (1.0f + __ldg(a.debye_table + 1 + 2 * m))), ld4(a.rd_state + (m * a.rd_pole + o)), z);
+            n = n - q_mul(Quad{cb0, cb1}, s0, z);
+            const Quad de = n - f, w = ld4(a.rd_dd + o);
+            for (int m = 0; m < poles; ++m) {
+                float* p = a.rd_state + (m * a.rd_pole + o);
+                const Quad b = q_bc(__ldg(a.debye_table + 1 + 2 * m)), c = q_bc(__ldg(a.debye_table + 2 + 2 * m));
+                st4(p, q_mul(b, ld4(p), z) + q_mul(q_mul(w, c, z), de, z));
+            }
+        }
     } else {
         n = f - q_mul(q_bc(a.k_mu), t, z);
         if (!S_J) {   // the row's last node has no k + 1 neighbour (the padding past it is 0 and stays 0)
@@ -369,33 +392,43 @@ struct ResWalk {
 // grid backwards: it starts on the planes the H half has just left in the L2, and the next H half on
 // those it leaves (of a grid whose state is more than the L2 keeps, a walk in one direction finds every
 // plane evicted: the adjoint sweep at 161x161x97 moved 218 MB a step through HBM; 93 -> 76 us a step).
-template <int C, int F, typename CID>
+template <int C, int F, typename CID, bool DEBYE>
 __device__ __forceinline__ void res_half(const ResArgs& a, const ResNode* X, const ResNode* Y, const float* Z, int np2, unsigned first,
                                          const float* src, const float* own, float* out, const float* psi_in, float* psi_out) {
     ResWalk<F != 0> at(a, first);
     // the E half's class ids a group ahead: its coefficients' addresses stand when its other loads start
     const CID* cls = static_cast<const CID*>(a.node_class);
     auto ids = [&](const ResWalk<F != 0>& w) { return res_load_ids(cls + (unsigned(w.row) * unsigned(a.g.p2) + unsigned(w.col) * 4u)); };
+    auto place = [&](const ResWalk<F != 0>& w) { return __ldg(a.rd_index + (w.row * int(a.quads.d) + w.col)); };
     IdWords<CID> words{};
-    if (F && at.inside(a)) words = ids(at);
+    int dg = -1;
+    if (F && at.inside(a)) {
+        words = ids(at);
+        if (DEBYE) dg = place(at);
+    }
     while (at.inside(a)) {
         ResWalk<F != 0> nx = at;
         nx.next(a);
         IdWords<CID> ahead{};
-        if (F && nx.inside(a)) ahead = ids(nx);
-        res_update<C, F, CID>(a, X, Y, Z, np2, unsigned(at.row), at.i, at.j, at.col * 4, words, src, own, out, psi_in, psi_out);
+        int dn = -1;
+        if (F && nx.inside(a)) {
+            ahead = ids(nx);
+            if (DEBYE) dn = place(nx);
+        }
+        res_update<C, F, CID, DEBYE>(a, X, Y, Z, np2, unsigned(at.row), at.i, at.j, at.col * 4, words, dg, src, own, out, psi_in, psi_out);
         at = nx;
         words = ahead;
+        dg = dn;
     }
 }
 
-template <int F, typename CID>
+template <int F, typename CID, bool DEBYE>
 __device__ __forceinline__ void res_field(const ResArgs& a, int comp, const ResNode* X, const ResNode* Y, const float* Z, int np2,
                                           unsigned first, const float* src, const float* own, float* out, const float* psi_in,
                                           float* psi_out) {
-    if (comp == 0) res_half<0, F, CID>(a, X, Y, Z, np2, first, src, own, out, psi_in, psi_out);
-    else if (comp == 1) res_half<1, F, CID>(a, X, Y, Z, np2, first, src, own, out, psi_in, psi_out);
-    else res_half<2, F, CID>(a, X, Y, Z, np2, first, src, own, out, psi_in, psi_out);
+    if (comp == 0) res_half<0, F, CID, DEBYE>(a, X, Y, Z, np2, first, src, own, out, psi_in, psi_out);
+    else if (comp == 1) res_half<1, F, CID, DEBYE>(a, X, Y, Z, np2, first, src, own, out, psi_in, psi_out);
+    else res_half<2, F, CID, DEBYE>(a, X, Y, Z, np2, first, src, own, out, psi_in, psi_out);
 }
 
 // A port's voltage (F = 0, E settled after step n) or current (F = 1, H of step n) into its series
@@ -488,7 +521,7 @@ __device__ __forceinline__ unsigned res_block_of(const ResArgs& a, long long f, 
 // 4-node groups, in row order, a third of its threads' number at a time in turn, three warps (one per
 // component) to 32 groups: a block's groups are whole rows (its j neighbours and the three components' shared loads are
 // mostly in its L1), and the layer's heavier groups fall on all blocks alike.
-template <typename CID, bool CLUSTER>
+template <typename CID, bool CLUSTER, bool DEBYE>
 __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_constant__ ResArgs a) {
     extern __shared__ __align__(16) float res_sm[];
     const Geom& g = a.g;
@@ -502,15 +535,19 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
     const unsigned groups = blockDim.x / 3u;
     const unsigned first = blockIdx.x * groups + unsigned(w / 3) * 32u + (threadIdx.x & 31u);   // the lane's first group
     const unsigned G = gridDim.x, b = blockIdx.x;
-    // the lists are shared out 32 entries at a time, one warp of every block before a block's next
-    const unsigned t = (unsigned(w) * G + b) * 32u + (threadIdx.x & 31u), nt = G * blockDim.x;
+    // the lists are shared out 32 entries at a time, one warp of every block before a block's next (formed
+    // where used, as the history's place is: the walks between need every register)
+    auto t = [] { return ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32u + (threadIdx.x & 31u); };
+    auto nt = [] { return gridDim.x * blockDim.x; };
+    auto place = [&](unsigned n) -> long long {   // step n's place in the design history, or -1
+        const long long v = (long long)n - *a.hist_base;
+        return v >= a.hist_cap ? -1 : v;
+    };
     const unsigned n0 = *(volatile const unsigned*)a.counter;
     int own = 0;   // a source or inductor edge among the block's nodes
     for (int q = threadIdx.x; q < a.ns; q += blockDim.x) own |= res_block_of(a, a.src[q].f, G, groups) == b;
     for (int q = threadIdx.x; q < a.ni; q += blockDim.x) own |= res_block_of(a, a.ind[q].f, G, groups) == b;
     own = __syncthreads_or(own);
-    const bool third = a.n_debye > 0 || a.n_design > 0;
-    const long long hist0 = a.n_design ? *a.hist_base : 0;
     unsigned target = 0;
     for (int s = 0; s <= a.steps; ++s) {
         const unsigned n = n0 + unsigned(s);
@@ -518,32 +555,29 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
         if (s > 0) {
             if (threadIdx.x < 32)
                 for (int p = int(G - 1 - b); p < a.n_ports; p += int(G)) res_probe<0>(a, p, n - 1);
-            if (a.plane) res_plane<0>(a, n - 1, t, nt);
-            if (a.ntff) res_ntff<0>(a, n - 1, t, nt);
+            if (a.plane) res_plane<0>(a, n - 1, t(), nt());
+            if (a.ntff) res_ntff<0>(a, n - 1, t(), nt());
         }
         if (s == a.steps) break;
         const float* e_in = s ? a.e : a.e_src;
-        long long slot = -1;   // this step's place in the design history
         if (a.n_design) {
-            slot = (long long)n - hist0;
-            if (slot >= a.hist_cap) slot = -1;
+            const long long slot = place(n);
+            if (slot >= 0)
+                for (int q = int(t()); q < a.n_design; q += int(nt())) {
+                    const int4 d = a.design[q];
+                    a.hist_e[slot * a.n_design + q] = e_in[d.x * g.cs + ((long long)d.y * g.n1 + d.z) * g.p2 + d.w];
+                }
         }
-        for (int q = int(t); q < a.n_debye; q += int(nt)) a.debye_old[q] = e_in[a.debye_f[q]];
-        if (slot >= 0)
-            for (int q = int(t); q < a.n_design; q += int(nt)) {
-                const int4 d = a.design[q];
-                a.hist_e[slot * a.n_design + q] = e_in[d.x * g.cs + ((long long)d.y * g.n1 + d.z) * g.p2 + d.w];
-            }
         // ... and the new H
         const float *h_in = s ? a.h : a.h_src, *p_in = s ? a.psi_h : a.psi_h_src;
-        res_field<0, CID>(a, comp, X, Y, Z, np2, first, e_in, h_in, a.h, p_in, a.psi_h);
+        res_field<0, CID, false>(a, comp, X, Y, Z, np2, first, e_in, h_in, a.h, p_in, a.psi_h);
         if (!res_barrier<CLUSTER>(a, target += G)) return;
         // ---- phase B: what reads the new H, and the new E
         if (threadIdx.x < 32)
             for (int p = int(G - 1 - b); p < a.n_ports; p += int(G)) res_probe<1>(a, p, n);
-        if (a.plane) res_plane<1>(a, n, t, nt);
-        if (a.ntff) res_ntff<1>(a, n, t, nt);
-        res_field<1, CID>(a, comp, X, Y, Z, np2, first, a.h, e_in, a.e, a.psi_e, a.psi_e);
+        if (a.plane) res_plane<1>(a, n, t(), nt());
+        if (a.ntff) res_ntff<1>(a, n, t(), nt());
+        res_field<1, CID, DEBYE>(a, comp, X, Y, Z, np2, first, a.h, e_in, a.e, a.psi_e, a.psi_e);
         if (own) {   // the source, then the inductors (lumped_block), on the block's own edges
             __syncthreads();
             const float p = n < a.sc.cap ? a.sc.pulse[n] : pulse_at(a.sc, (float(n) + 0.5f) * a.sc.dt);
@@ -562,30 +596,64 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
             }
         }
         if (!res_barrier<CLUSTER>(a, target += G)) return;
-        if (third) {
-            // ---- phase C: the Debye ADE (k_debye_post_cb; its edges carry no source or element) and
-            // the design edges' curl terms (k_design_record)
-            const int poles = a.n_debye ? int(a.debye_table[0]) : 0;
-            for (int q = int(t); q < a.n_debye; q += int(nt)) {
-                const long long fi = a.debye_f[q];
-                float s0 = 0.0f;
-                for (int k = 0; k < poles; ++k)
-                    s0 += 0.5f * (1.0f + a.debye_table[1 + 2 * k]) * a.debye_state[(long long)k * a.n_debye + q];
-                const float next = a.e[fi] - a.debye_cb[q] * s0;
-                a.e[fi] = next;
-                const float de = next - a.debye_old[q], w = a.debye_dd[q];
-                for (int k = 0; k < poles; ++k) {
-                    const long long p = (long long)k * a.n_debye + q;
-                    a.debye_state[p] = a.debye_table[1 + 2 * k] * a.debye_state[p] + w * a.debye_table[2 + 2 * k] * de;
-                }
-            }
+        if (a.n_design) {
+            // ---- phase C: the design edges' curl terms (k_design_record)
+            const long long slot = place(n);
             if (slot >= 0)
-                for (int q = int(t); q < a.n_design; q += int(nt))
+                for (int q = int(t()); q < a.n_design; q += int(nt()))
                     a.hist_s[slot * a.n_design + q] = design_curl(g, a.design[q], a.h, a.psi_e);
             if (!res_barrier<CLUSTER>(a, target += G)) return;
         }
     }
-    if (t == 0) *a.counter = n0 + unsigned(a.steps);
+    if (t() == 0) *a.counter = n0 + unsigned(a.steps);
+}
+
+// ---- the Debye layout by groups, from the edge list
+
+struct RdMap {
+    Geom g;
+    unsigned quads;          // groups per row
+    const long long* f;      // the list
+    int count;
+    int* index;
+};
+__device__ __forceinline__ unsigned rd_group(const RdMap& m, int q, unsigned& at) {
+    const long long f = m.f[q];
+    const int c = int(f / m.g.cs);
+    const long long id = f - c * m.g.cs, row = id / m.g.p2;
+    const unsigned k = unsigned(id - row * m.g.p2);
+    at = 4u * unsigned(c) + (k & 3u);
+    return unsigned(row) * m.quads + k / 4u;
+}
+__global__ void k_rd_mark(RdMap m) {
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m.count; q += gridDim.x * blockDim.x) {
+        unsigned at;
+        m.index[rd_group(m, q, at)] = 1;
+    }
+}
+// flags and their running sums to places
+__global__ void k_rd_places(int* index, const int* sums, unsigned n) {
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) index[q] = index[q] ? sums[q] : -1;
+}
+__global__ void k_rd_weights(RdMap m, const float* __restrict__ dd, float* __restrict__ out) {
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m.count; q += gridDim.x * blockDim.x) {
+        unsigned at;
+        const unsigned g = rd_group(m, q, at);
+        out[unsigned(m.index[g]) * 12u + at] = dd[q];
+    }
+}
+// The pole states between the list and the groups (TO: to the groups).
+template <bool TO>
+__global__ void k_rd_move(RdMap m, int poles, unsigned pole, float* list, float* dense) {
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m.count; q += gridDim.x * blockDim.x) {
+        unsigned at;
+        const unsigned g = rd_group(m, q, at), o = unsigned(m.index[g]) * 12u + at;
+        for (int k = 0; k < poles; ++k) {
+            float &l = list[(long long)k * m.count + q], &d = dense[(size_t)k * pole + o];
+            if (TO) d = l;
+            else l = d;
+        }
+    }
 }
 
 }  // namespace fg

@@ -49,10 +49,11 @@ def test_the_resident_sweep_equals_the_separate_transposes(gpu, monkeypatch, dim
         assert np.array_equal(a.grad_sigma, other.grad_sigma)
 
 
-def test_a_history_larger_than_the_checkpoints_is_run_again(gpu):
+@pytest.mark.parametrize("debye", [False, True])
+def test_a_history_larger_than_the_checkpoints_is_run_again(gpu, debye):
     """A design that fills much of the grid: its whole history would take more than two checkpoints, so
     the segments run again, with the gradient of the stored history."""
-    scene, spec, _, _ = W.flux_design(30, 30, 32, pml=4, design=(16, 16, 8), steps=240, checkpoints=4)
+    scene, spec, _, _ = W.flux_design(30, 30, 32, pml=4, design=(16, 16, 8), steps=240, checkpoints=4, debye=debye)
     sc = scene()
     sim = fdtd.Sim.try_new(*sc.args())
     b = fdtd.flux_gradient(gpu, sim, 0, sc.pulse, spec)
