@@ -7,7 +7,8 @@
 // triangles (the reference's hierarchy, bvh.rs): a warp takes a triangle, tests the few columns under its
 // bounding box with the reference's own hit test, and counts, then stores, each crossing in its column's
 // list; a thread per column sorts its list and walks it as repeated nearest-crossing queries would. Work
-// goes with the crossings, no hierarchy is built on the host (it was half of a fill), and no thread
+// goes with the crossings, no hierarchy is built on the host (it was half of a fill; only a mesh whose
+// hits it could prune needs its boxes, see Boxes), and no thread
 // chases a tree through memory once per crossing: 12,288 triangles onto 160x128x96 cells take 6.9 ms a
 // fill with its copies, 15.4 before.
 // sheet_edges runs one block per triangle over the nodes near it. Every mark is a byte store of 1, so
@@ -32,6 +33,46 @@ namespace fg {
 namespace raster {
 
 constexpr int MAX_CROSSINGS = 1 << 20;     // per column
+
+// The boxes that Bvh::build (bvh.rs:62-93: median splits along the longest axis, leaves of at most 4
+// triangles) gives each triangle's leaf. The hit test takes a ray up to a 1e-9 part of the triangle outside
+// of it, and the rays pass a 1e-6 part of a cell from the grid's lines: past the edge of a face more than
+// some 1200 cells wide a ray can hit, and whether it counts is for the leaf's box to say (a triangle's own
+// box never tells more than its leaf's, which holds it).
+struct Boxes {
+    const double* tri;
+    std::vector<int> order;
+    std::vector<double> out;   // per triangle: low, high
+
+    Boxes(const double* t, size_t n) : tri(t), order(n), out(n * 6) {
+        for (size_t q = 0; q < n; ++q) order[q] = int(q);
+        split(0, int(n));
+    }
+    double centre(int i, int axis) const {
+        const double* t = tri + size_t(i) * 9;
+        return (t[axis] + t[3 + axis] + t[6 + axis]) / 3.0;
+    }
+    void split(int start, int end) {
+        double b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        for (int q = start; q < end; ++q)
+            for (int c = 0; c < 9; ++c) {
+                const double v = tri[size_t(order[size_t(q)]) * 9 + size_t(c)];
+                b[c % 3] = std::fmin(b[c % 3], v);
+                b[3 + c % 3] = std::fmax(b[3 + c % 3], v);
+            }
+        if (end - start <= 4) {
+            for (int q = start; q < end; ++q) std::copy(b, b + 6, &out[size_t(order[size_t(q)]) * 6]);
+            return;
+        }
+        const double ex[3] = {b[3] - b[0], b[4] - b[1], b[5] - b[2]};
+        const int axis = (ex[0] >= ex[1] && ex[0] >= ex[2]) ? 0 : (ex[1] >= ex[2] ? 1 : 2);
+        const int middle = (start + end) / 2;
+        std::nth_element(order.begin() + start, order.begin() + middle, order.begin() + end,
+                         [&](int x, int y) { return centre(x, axis) < centre(y, axis); });
+        split(start, middle);
+        split(middle, end);
+    }
+};
 
 __device__ __forceinline__ void dsub(const double* a, const double* b, double* o) {
     o[0] = a[0] - b[0]; o[1] = a[1] - b[1]; o[2] = a[2] - b[2];
@@ -122,18 +163,22 @@ __device__ __forceinline__ void span_under(const double* line, int n, double shi
 }
 
 // The crossings of one axis's columns: a warp per triangle (and part of its columns, blockIdx.y). STORE
-// false: counted per column; true: stored in the columns [c0, c1)' lists, at offset[col] - base on.
+// false: counted per column; true: stored in the columns [c0, c1)' lists, at offset[col] - base on. A hit
+// beside its triangle's box counts if the ray passes through its leaf's (`leaf`; null: *stray says there is one).
 template <bool STORE>
 __global__ void k_crossings(FillAxis f, const double* tri, long long ntri, unsigned long long* count,
-                            const unsigned long long* offset, double* hits, unsigned long long base, long long c0, long long c1) {
+                            const unsigned long long* offset, double* hits, unsigned long long base, long long c0, long long c1,
+                            const double* leaf, int* stray) {
     const long long ti = blockIdx.x * (long long)(blockDim.x / 32) + (threadIdx.x >> 5);
     if (ti >= ntri) return;
     const double* t = tri + ti * 9;
     int a[2], b[2];
+    double lo[2], hi[2];
     for (int x = 0; x < 2; ++x) {
         const int ax = x ? f.v : f.u;
-        const double lo = fmin(fmin(t[ax], t[3 + ax]), t[6 + ax]), hi = fmax(fmax(t[ax], t[3 + ax]), t[6 + ax]);
-        span_under(f.line[ax], f.n[ax], f.step[ax] * (x ? 2.345678e-6 : 1.234567e-6), f.step[ax], lo, hi, a[x], b[x]);
+        lo[x] = fmin(fmin(t[ax], t[3 + ax]), t[6 + ax]);
+        hi[x] = fmax(fmax(t[ax], t[3 + ax]), t[6 + ax]);
+        span_under(f.line[ax], f.n[ax], f.step[ax] * (x ? 2.345678e-6 : 1.234567e-6), f.step[ax], lo[x], hi[x], a[x], b[x]);
     }
     a[0] = max(a[0] - f.us, 0);
     b[0] = min(b[0] - f.us, f.wide);
@@ -151,6 +196,16 @@ __global__ void k_crossings(FillAxis f, const double* tri, long long ntri, unsig
         column_ray(f, col, cell, from);
         const double x = hit(t, from, dir);
         if (!(x > 0.0) || !(x < INFINITY)) continue;   // NaN: no crossing
+        const double o0 = from[f.u], o1 = from[f.v];
+        if (!(lo[0] < o0 && o0 < hi[0] && lo[1] < o1 && o1 < hi[1])) {
+            if (leaf) {   // the slab test of bvh.rs:95-110 across the ray (a side the ray runs along is outside, a flat box in)
+                const double* b6 = leaf + ti * 6;
+                auto in = [&](int ax, double o) { return (b6[ax] < o && o < b6[3 + ax]) || (b6[ax] == o && o == b6[3 + ax]); };
+                if (!in(f.u, o0) || !in(f.v, o1)) continue;
+            } else {
+                *stray = 1;
+            }
+        }
         const unsigned long long at = atomicAdd(count + col, 1ull);
         if (STORE) hits[offset[col] - base + at] = x;
     }
@@ -419,7 +474,7 @@ int raster_fill(Gpu* gpu, const double* tris, uint64_t ntri, const std::vector<d
     cudaStream_t st;
     RS_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     struct Bufs {
-        void* p[2] = {};
+        void* p[3] = {};
         cudaStream_t st;
         ~Bufs() {
             cudaStreamSynchronize(st);
@@ -457,13 +512,30 @@ int raster_fill(Gpu* gpu, const double* tris, uint64_t ntri, const std::vector<d
     }
     RS_CUDA(cudaMemsetAsync(d_in, 0, sizes[2] + sizes[3] + sizes[4] + sizes[5], st));
     const dim3 grid(unsigned((ntri + 3) / 4), unsigned(std::min<uint64_t>(64, std::max<uint64_t>(1, 148 * 16 / ((ntri + 3) / 4)))));
-    for (int a = 0; a < 3; ++a)
-        k_crossings<false><<<grid, 128, 0, st>>>(f[a], tri, (long long)ntri, count + col0[a], nullptr, nullptr, 0, 0, cols[a]);
-    RS_CUDA(cudaGetLastError());
-    RS_CUDA(cub::DeviceScan::ExclusiveSum(part[7], scan, count, offset, (long long)(nc + 1), st));
     unsigned long long crossings = 0;
-    RS_CUDA(cudaMemcpyAsync(&crossings, offset + nc, 8, cudaMemcpyDeviceToHost, st));
+    const double* leaf = nullptr;
+    auto count_all = [&]() -> int {   // each column's crossings, where its list starts, and whether a hit was a stray
+        for (int a = 0; a < 3; ++a)
+            k_crossings<false><<<grid, 128, 0, st>>>(f[a], tri, (long long)ntri, count + col0[a], nullptr, nullptr, 0, 0, cols[a], leaf,
+                                                     d_err + 1);
+        RS_CUDA(cudaGetLastError());
+        RS_CUDA(cub::DeviceScan::ExclusiveSum(part[7], scan, count, offset, (long long)(nc + 1), st));
+        RS_CUDA(cudaMemcpyAsync(&crossings, offset + nc, 8, cudaMemcpyDeviceToHost, st));
+        return FG_OK;
+    };
+    int stray = 0, rc = count_all();
+    if (rc) return rc;
+    RS_CUDA(cudaMemcpyAsync(&stray, d_err + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     RS_CUDA(cudaStreamSynchronize(st));
+    if (stray) {
+        const Boxes boxes(tris, size_t(ntri));
+        RS_CUDA(cudaMalloc(&m.p[2], size_t(ntri) * 48));
+        RS_CUDA(cudaMemcpyAsync(m.p[2], boxes.out.data(), size_t(ntri) * 48, cudaMemcpyHostToDevice, st));
+        leaf = static_cast<const double*>(m.p[2]);
+        RS_CUDA(cudaMemsetAsync(count, 0, (nc + 1) * 8, st));
+        if ((rc = count_all())) return rc;
+        RS_CUDA(cudaStreamSynchronize(st));
+    }
     // the columns in runs whose lists fit the room: all at once for an ordinary mesh, else at most 2^26
     // crossings (or one column's) at a time
     struct Piece { int axis; long long c0, c1; unsigned long long base; };
@@ -489,7 +561,8 @@ int raster_fill(Gpu* gpu, const double* tris, uint64_t ntri, const std::vector<d
     RS_CUDA(cudaMemsetAsync(count, 0, nc * 8, st));   // counted again as the lists fill
     for (const Piece& p : pieces) {
         const long long o = col0[p.axis];
-        k_crossings<true><<<grid, 128, 0, st>>>(f[p.axis], tri, (long long)ntri, count + o, offset + o, hits, p.base, p.c0, p.c1);
+        k_crossings<true><<<grid, 128, 0, st>>>(f[p.axis], tri, (long long)ntri, count + o, offset + o, hits, p.base, p.c0, p.c1, leaf,
+                                                d_err + 1);
         k_fill_axis<<<unsigned((p.c1 - p.c0 + 127) / 128), 128, 0, st>>>(f[p.axis], count + o, offset + o, hits, p.base, p.c0, p.c1,
                                                                        d_in, d_thin, d_err);
     }

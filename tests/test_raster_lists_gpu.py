@@ -33,3 +33,20 @@ def test_fill_with_long_short_and_wide_lists_equals_the_oracle(gpu, mesh, lines)
     assert np.array_equal(got.inside, np.nonzero(inside)[0])
     assert np.array_equal(got.thin, np.nonzero(thin)[0])
     assert len(got.inside) + len(got.thin) > 0
+
+
+@pytest.mark.parametrize("cells", [700, 1400])
+def test_rays_just_past_the_edge_of_a_wide_face_stay_outside(gpu, cells):
+    """The rays run 1.2e-6 of a cell past the box's far edges, within the hit test's 1e-9 of a triangle 1400
+    cells wide; the mesh's boxes keep them out, so a face of two triangles fills as one of many short ones."""
+    lo, hi = np.array([1.0, 1.0, 1.0]), np.array([cells + 1.0, 5.0, 4.0])
+    wide = cuboid(lo, hi)
+    parts = np.linspace(lo[0], hi[0], 15)
+    short = np.concatenate([cuboid([a, lo[1], lo[2]], [b, hi[1], hi[2]]) for a, b in zip(parts[:-1], parts[1:])])
+    x = short.reshape(-1, 3, 3)[..., 0]
+    inner = (x == x[:, :1]).all(axis=1) & (x[:, 0] > lo[0]) & (x[:, 0] < hi[0])    # the walls between the parts
+    short = short.reshape(-1, 3, 3)[~inner]
+    samples = [np.arange(n, dtype=float) for n in (cells + 3, 7, 6)]
+    a, b = R.fill(gpu, wide, samples, "ijk"), R.fill(gpu, short, samples, "ijk")
+    assert np.array_equal(a.inside, b.inside) and np.array_equal(a.thin, b.thin)
+    assert len(a.inside) > 0
