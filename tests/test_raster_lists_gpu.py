@@ -35,18 +35,28 @@ def test_fill_with_long_short_and_wide_lists_equals_the_oracle(gpu, mesh, lines)
     assert len(got.inside) + len(got.thin) > 0
 
 
-@pytest.mark.parametrize("cells", [700, 1400])
-def test_rays_just_past_the_edge_of_a_wide_face_stay_outside(gpu, cells):
-    """The rays run 1.2e-6 of a cell past the box's far edges, within the hit test's 1e-9 of a triangle 1400
-    cells wide; the mesh's boxes keep them out, so a face of two triangles fills as one of many short ones."""
-    lo, hi = np.array([1.0, 1.0, 1.0]), np.array([cells + 1.0, 5.0, 4.0])
-    wide = cuboid(lo, hi)
-    parts = np.linspace(lo[0], hi[0], 15)
-    short = np.concatenate([cuboid([a, lo[1], lo[2]], [b, hi[1], hi[2]]) for a, b in zip(parts[:-1], parts[1:])])
-    x = short.reshape(-1, 3, 3)[..., 0]
-    inner = (x == x[:, :1]).all(axis=1) & (x[:, 0] > lo[0]) & (x[:, 0] < hi[0])    # the walls between the parts
-    short = short.reshape(-1, 3, 3)[~inner]
-    samples = [np.arange(n, dtype=float) for n in (cells + 3, 7, 6)]
-    a, b = R.fill(gpu, wide, samples, "ijk"), R.fill(gpu, short, samples, "ijk")
-    assert np.array_equal(a.inside, b.inside) and np.array_equal(a.thin, b.thin)
-    assert len(a.inside) > 0
+def _pieces(lo, hi, axis, parts):
+    """The cuboid's surface with the faces along `axis` cut into `parts`."""
+    cuts, out = np.linspace(lo[axis], hi[axis], parts + 1), []
+    for a, b in zip(cuts[:-1], cuts[1:]):
+        l, h = lo.copy(), hi.copy()
+        l[axis], h[axis] = a, b
+        out.append(cuboid(l, h))
+    t = np.concatenate(out).reshape(-1, 3, 3)
+    x = t[..., axis]
+    return t[~((x == x[:, :1]).all(axis=1) & (x[:, 0] > lo[axis]) & (x[:, 0] < hi[axis]))]
+
+
+@pytest.mark.parametrize("axis,cells", [(0, 1400), (1, 700), (1, 1400), (2, 1400)])
+def test_rays_just_past_the_edge_of_a_wide_face_stay_outside(gpu, axis, cells):
+    """The rays run 1.2e-6 of a cell past the box's far edges: within the hit test's 1e-9 of a triangle 1400
+    cells wide (along y it fills 30 nodes too many), where the mesh's boxes keep them out. So a box fills as
+    one whose faces are short pieces, which no such ray hits."""
+    n = [7, 6, 9]
+    n[axis] = cells + 3
+    lo, hi = np.ones(3), np.array(n) - 2.0
+    samples = [np.arange(k, dtype=float) for k in n]
+    wide, short = (R.fill(gpu, m, samples, "ijk") for m in (cuboid(lo, hi), _pieces(lo, hi, axis, 14)))
+    inside, _ = O.raster_fill(_pieces(lo, hi, axis, 14), samples, n, 0)
+    assert np.array_equal(wide.inside, short.inside) and np.array_equal(wide.thin, short.thin)
+    assert np.array_equal(wide.inside, np.nonzero(inside)[0]) and len(wide.inside) > 0
