@@ -81,9 +81,12 @@ __device__ __forceinline__ KNode k_node(const KAxis& kx, int k) {
 __device__ __forceinline__ float cpml_term(float b, float psi, float c, float d, float raw) { return b * psi + c * d * raw; }
 
 constexpr int SHELL_THREADS = 256;   // 8 rows per block
-// k_shell_h is held to 64 registers (4 blocks per SM, 32 warps: a few bytes spill) for more loads in
-// flight: 10 % faster at 512^3 than at its natural 80 registers (3 blocks); k_shell_e at 64 was 3 %
-// slower and keeps its 80.
+// Both are held to 64 registers (4 blocks per SM, 32 warps: a few bytes spill) for more loads in flight.
+// k_shell_h: 10 % faster at 512^3 than at its natural 80 registers (3 blocks). k_shell_e: 196 us at 80
+// registers with psi loaded for the live edges only, two dependent loads (class id, class) behind the
+// rest; 180 with psi loaded at once, 171 at 64 registers on top (583 MB, 3.4 TB/s; the merged batch launch, 112
+// registers before: 851 -> 800 us a step of 12 grids); class ids a row's
+// pass ahead cost registers (254 at 2 blocks per SM, 174 at 3, 181 at 4).
 
 // The new H of one row of shell nodes (cpu.rs:48-107): H_c = H_c - k_mu [(dE_v/du) inv_d_u + psi_u
 // - (dE_u/dv) inv_d_v - psi_v], each psi_a updated where the node's slot along a is live. All loads
@@ -190,10 +193,11 @@ __device__ __forceinline__ void shell_e_row(const Geom& g, const ShellRows& b, c
         const long long o0j = g.psi_off[0 * 3 + 1] + py + k, o0k = g.psi_off[0 * 3 + 2] + pz + ak.slot;
         const long long o1k = g.psi_off[1 * 3 + 2] + pz + ak.slot, o1i = g.psi_off[1 * 3 + 0] + px + k;
         const long long o2i = g.psi_off[2 * 3 + 0] + px + k, o2j = g.psi_off[2 * 3 + 1] + py + k;
+        // not for the live edges alone: those are known one load (the class's) after the ids
         const bool lj = aj.slot_e >= 0, lk = ak.slot >= 0, li = ai.slot_e >= 0;
-        const float s0j = run0 && lj ? psi[o0j] : 0.f, s0k = run0 && lk ? pz_in[o0k] : 0.f;
-        const float s1k = run1 && lk ? pz_in[o1k] : 0.f, s1i = run1 && li ? psi[o1i] : 0.f;
-        const float s2i = run2 && li ? psi[o2i] : 0.f, s2j = run2 && lj ? psi[o2j] : 0.f;
+        const float s0j = lj ? psi[o0j] : 0.f, s0k = lk ? pz_in[o0k] : 0.f;
+        const float s1k = lk ? pz_in[o1k] : 0.f, s1i = li ? psi[o1i] : 0.f;
+        const float s2i = li ? psi[o2i] : 0.f, s2j = lj ? psi[o2j] : 0.f;
         if (run0) {   // Ex: U = j, V = k
             const float hv = hz - hz_j, hu = hy - hy_k;
             float t1 = hv * aj.inv_dd, t2 = hu * ak.inv;
@@ -248,7 +252,7 @@ __global__ void __launch_bounds__(SHELL_SIDE_THREADS, 8) k_shell_h_side(Geom g, 
 }
 
 template <typename CID>
-__global__ void __launch_bounds__(SHELL_THREADS) k_shell_e(Geom g, ShellRows b, KAxis kx, const CID* __restrict__ node_class,
+__global__ void __launch_bounds__(SHELL_THREADS, 4) k_shell_e(Geom g, ShellRows b, KAxis kx, const CID* __restrict__ node_class,
                                                            const DevCoef* __restrict__ classes,
                                                            const float* __restrict__ h, const float* __restrict__ e_in,
                                                            float* __restrict__ e_out, float* __restrict__ psi,
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(SHELL_THREADS, 4) k_batch_shell_h(const ShellG
 }
 
 template <typename CID>
-__global__ void __launch_bounds__(SHELL_THREADS) k_batch_shell_e(const ShellGrid* __restrict__ grids,
+__global__ void __launch_bounds__(SHELL_THREADS, 4) k_batch_shell_e(const ShellGrid* __restrict__ grids,
                                                               const int* __restrict__ block_grid, int parity) {
     const ShellGrid& G = grids[block_grid[blockIdx.x]];
     const unsigned r = unsigned(int(blockIdx.x) - G.block0) * (SHELL_THREADS / 32) + (threadIdx.x >> 5);
