@@ -852,8 +852,6 @@ bool resident_allowed(const Session& s) {
            s.stall_plane < 0 && s.n_wires == 0 && s.n_sheets == 0;
 }
 
-// Whether a session's steps run resident, and its launch shape, with room on each SM for the blocks of
-// `share` such launches (of sessions stepped side by side).
 template <typename F>
 int with_adj_resident(int cid_bytes, bool cluster, F&& f) {
     if (cid_bytes == 1) return cluster ? f(k_adj_resident<uint8_t, true>) : f(k_adj_resident<uint8_t, false>);
@@ -861,6 +859,8 @@ int with_adj_resident(int cid_bytes, bool cluster, F&& f) {
     return cluster ? f(k_adj_resident<uint32_t, true>) : f(k_adj_resident<uint32_t, false>);
 }
 
+// Whether a session's steps run resident, and its launch shape, with room on each SM for the blocks of
+// `share` such launches (of sessions stepped side by side).
 int plan_resident(Session& s, int share, std::string& err) {
     const Geom& g = s.geom;
     s.resident = false;

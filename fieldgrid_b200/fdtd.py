@@ -584,7 +584,8 @@ class FluxSpec:
     dA (Ex^ conj(Hy^) - Ey^ conj(Hx^)) at `freq`, and the design box of cells [lo, hi) whose
     relative permittivity and conductivity the gradient is over. `window` None: the nodes inside
     the CPML. `checkpoints` 0 keeps every step's design-edge history; c > 0 keeps about c field
-    checkpoints and re-runs each segment in the backward sweep."""
+    checkpoints and re-runs each segment in the backward sweep, unless the whole history takes no
+    more memory than they would."""
     design_lo: tuple
     design_hi: tuple
     plane_k: int
@@ -694,7 +695,9 @@ def flux_gradient_batch(g, sims, pulses, specs, driven=None, group: int = 16) ->
 
 class Batch:
     """Many Sims stepped together: one persistent work-list launch marches every grid per step,
-    then one launch each for all grids' Debye edges, sources and probes, in a captured graph.
+    then one launch each for all grids' Debye edges, sources and probes, in a captured graph; or each
+    grid on a graph branch of its own, merged march and shell launches, or many steps of one grid in
+    one launch (`tile` 3 to 6).
     `tune` times the candidate shapes first (tile, persistent blocks per SM, planes per item) and
     keeps the fastest. Each grid's results equal stepping it alone with the fused step."""
 

@@ -1,5 +1,5 @@
-"""Mesh -> grid rasterisation (`sims_field::raster`, crates/sims-field/src/raster.rs, over the
-hierarchy of bvh.rs) on the CUDA engine: `fill`, `solid_edges`, `solid_cells`, `sheet_edges` and
+"""Mesh -> grid rasterisation (`sims_field::raster`, crates/sims-field/src/raster.rs,
+without a hierarchy) on the CUDA engine: `fill`, `solid_edges`, `solid_cells`, `sheet_edges` and
 `closed`, with the reference's names and argument meaning. Triangles are any array-like of shape
 (n, 3, 3) (vertex, coordinate) in f64; the ray casts and the sheet sweep run on the GPU (a `Gpu`
 must be given: there is no CPU path), `closed` on the host.

@@ -279,7 +279,10 @@ int fg_port_spectra(const float* series, uint64_t steps, uint64_t ports, uint64_
  * exact for the f32 update as the device runs it (a discrete adjoint), from one forward run on the
  * fused step and one backward sweep. checkpoints = 0 keeps each step's E and curl term on the
  * design edges; checkpoints = c keeps the full field state at the start of about c segments and
- * re-runs each segment before sweeping it (sqrt(steps) checkpoints: segment recomputation).
+ * re-runs each segment before sweeping it (sqrt(steps) checkpoints: segment recomputation), unless
+ * every step's history takes no more memory than those c states and a segment's history would: then
+ * it is kept and nothing re-runs (fg_flux_result's segments and segment_len then still say what the
+ * checkpoints asked for).
  * The design box must stay off the grid boundary and off PEC, lumped, port and Debye edges; the
  * Sim may hold Debye media outside the design box (their ADE is transposed in the backward sweep
  * and carried by the checkpoints), but no inductors, thin wires or resistive sheets. */
@@ -328,19 +331,23 @@ int fg_flux_gradient_batch(fg_gpu* g, const fg_sim* const* sims, const uint64_t*
  * grids' Debye edges, sources and port probes, captured in a CUDA graph; or (tile 3) one graph
  * branch per grid, each running that grid's own fused step on its stream, concurrently; or (tile 5)
  * one launch of the TMA march over every grid's clean box and one of each CPML shell kernel over
- * every grid's shell, then the shared Debye, source and probe launches. Each
+ * every grid's shell, then the shared Debye, source and probe launches; or (tile 6) each grid many
+ * steps in one launch with its state in L2, grid after grid. Each
  * grid's results are those of stepping it alone (fused step). Grids with thin wires or resistive
  * sheets, or that ask for a plane DFT or NTFF, are refused. With tune = 1 the batch times each
  * candidate (work-list tile 32x8, 64x4 or 32x4 with its persistent blocks per SM and x-planes per
- * work item, both kinds of graph branches and the merged launches) as a captured graph of a few steps, keeps the fastest and
- * resets every grid to step 0; with tune = 0 it uses the shape given. */
+ * work item, both kinds of graph branches, the merged launches and the resident grids) as a captured graph
+ * of a few steps, keeps the fastest and resets every grid to step 0; with tune = 0 it uses the shape given. */
 typedef struct fg_batch fg_batch;
 typedef struct fg_batch_options {
     int tune;
     int tile;                /* work-list march 0: 32x8, 1: 64x4, 2: 32x4 (k x j); 3: graph branches;
                                 4: graph branches, the grids of fewer than seg thousand nodes (all: seg 0)
                                 with the direct-load march (one launch per grid-step); 5: merged TMA march
-                                and shell launches over all grids */
+                                and shell launches over all grids; 6: the grids one after another, many
+                                steps a launch, blocks_per_sm (1 to 4) launches side by side, calls of
+                                fewer than 8 steps as 3; as 5 where a grid cannot step so (more than 23 M
+                                nodes) */
     int blocks_per_sm;       /* 0: the occupancy limit */
     int seg;                 /* x-planes per work item; 0: 32 */
     int graph_steps;         /* steps per captured graph; 0: 10 */
