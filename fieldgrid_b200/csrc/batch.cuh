@@ -629,8 +629,12 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
     if (!tune && fixed.tile == BATCH_RESIDENT) {
         share = std::min(std::max(fixed.blocks_per_sm, 1), 4);
         if ((rc = batch_plan_resident(*B, share, err))) return rc;
-        if (!B->resident_ok) { err = "a grid of this batch does not step resident"; return FG_ERR_INVALID; }
-        best = BatchShape{BATCH_BRANCHES, 0, 0};
+        if (B->resident_ok) {
+            best = BatchShape{BATCH_BRANCHES, 0, 0};
+        } else {   // a grid that cannot: the merged launches, as any number past theirs always chose
+            share = 0;
+            best.tile = BATCH_MERGED;
+        }
     }
     if (tune) {
         cudaEvent_t e0, e1;
@@ -707,7 +711,7 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
 int batch_new_c(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vector<RunSpec>& specs, bool tune,
                 int tile, int blocks_per_sm, int seg, int graph_steps, Batch** out, std::string& err) {
     BatchShape sh;
-    sh.tile = std::min(std::max(tile, 0), BATCH_RESIDENT);
+    sh.tile = tile == BATCH_RESIDENT ? tile : std::min(std::max(tile, 0), BATCH_MERGED);
     sh.blocks_per_sm = std::max(blocks_per_sm, 0);
     sh.seg = seg > 0 ? seg : 32;
     return batch_new(gpu, sims, specs, tune, sh, graph_steps > 0 ? graph_steps : 10, out, err);

@@ -29,7 +29,17 @@ def test_resident_grids_step_as_alone(gpu, monkeypatch, share):
     b.close()
 
 
-def test_a_grid_that_cannot_step_resident_is_refused(gpu):
+@pytest.mark.parametrize("tile", [6, 7])
+def test_a_grid_that_cannot_step_resident_takes_the_merged_launches(gpu, tile):
     sc = W.spheres(12, pml=5, count=2, rmin=1, rmax=2, steps=10)   # both layers in one 4-node group along k
-    with pytest.raises(fdtd.FdtdError, match="does not step resident"):
-        fdtd.Batch(gpu, [fdtd.Sim.try_new(*sc.args())], [sc.pulse], 10, tune=False, tile=6)
+    sim = fdtd.Sim.try_new(*sc.args())
+    b = fdtd.Batch(gpu, [sim], [sc.pulse], 10, tune=False, tile=tile)
+    assert b.info()["tile"] == "merged TMA launches"
+    b.step(10)
+    s = fdtd.Session(gpu, sim, 0, sc.pulse, sc.extras)
+    s.step(10)
+    n = 3 * int(np.prod(sc.grid.dims()))
+    for which in ("e", "h"):
+        assert np.array_equal(b.read(0, which, n), s.read(which, n))
+    s.close()
+    b.close()
