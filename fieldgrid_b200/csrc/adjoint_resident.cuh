@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_adj_resident(const __grid_co
     const unsigned first = b * groups + unsigned(w / 3) * 32u + (threadIdx.x & 31u);
     auto t = [] { return int(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32u + (threadIdx.x & 31u)); };   // k_resident's
     auto nt = [] { return int(gridDim.x * blockDim.x); };
-    unsigned target = 0;
+    unsigned target = a.late;
     for (long long n = A.n_hi - 1; n >= A.n_hi - a.steps; --n) {
         if (a.n_debye) {
             for (int q = t(); q < a.n_debye; q += nt()) {

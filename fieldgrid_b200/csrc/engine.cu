@@ -301,6 +301,8 @@ struct Session {
     // from FIELDGRID_TEST_WAIT_NS / FIELDGRID_TEST_STALL_PLANE, which only the failure-path test sets
     unsigned long long wait_ns = tma::WAIT_LIMIT_NS;
     int stall_plane = -1;
+    bool stall_barrier = false;     // test knob of the resident kernels' grid barrier (ResArgs::late)
+    bool unchecked = false;         // steps enqueued since the error word was last read
     int2* tma_own = nullptr;        // per block of the one-step march: the rows it writes
     // ---- the two-step mode (stencil_tb2.cuh). Step t reads field set, z-slab psi slot and Debye
     // state slot t mod 3 and writes (t + 1) mod 3; the x/y slabs keep the one-step scheme (E in
@@ -875,7 +877,7 @@ int plan_resident(Session& s, int share, std::string& err) {
         const long long even = ((total + blocks * passes - 1) / (blocks * passes) + 31) / 32 * 32;   // passes of one size
         return int(std::min(most, std::max<long long>(32, passes <= 4 ? even : most)));
     };
-    s.res_cluster = total <= RES_CLUSTER_GROUPS;
+    s.res_cluster = total <= RES_CLUSTER_GROUPS && !s.stall_barrier;   // the cluster's own barrier cannot run out
     const int most = s.res_cluster ? RES_CLUSTER : sms;
     s.res_groups = groups_of(most);
     s.res_blocks = s.res_cluster ? RES_CLUSTER : int(std::min<long long>(sms, (total + s.res_groups - 1) / s.res_groups));
@@ -910,6 +912,7 @@ void resident_shape(const Session& s, ResArgs& a) {
     a.bar = s.res_bar;
     a.error = s.error;
     a.wait_ns = s.wait_ns;
+    a.late = s.stall_barrier ? 1u : 0u;
     const unsigned q = unsigned(g.n2 + 3) / 4, pass = unsigned(s.res_blocks) * unsigned(s.res_groups);
     a.quads = FastDiv(q);
     a.rows = FastDiv(unsigned(g.n1));
@@ -2225,6 +2228,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
         s->wait_ns = std::min<unsigned long long>(std::max<unsigned long long>(std::strtoull(v, nullptr, 10),
                                                                                tma::WAIT_LIMIT_MIN_NS), tma::WAIT_LIMIT_NS);
     if (const char* v = std::getenv("FIELDGRID_TEST_STALL_PLANE")) s->stall_plane = std::atoi(v);
+    if (const char* v = std::getenv("FIELDGRID_TEST_STALL_BARRIER")) s->stall_barrier = v[0] == '1';
     plan_tma(*s);
     clk.mark("tma_maps");
     if (sp.ok && s->tma.ok && s->local) {
@@ -2391,6 +2395,7 @@ int session_reset(Session* s, std::string& err) {
 int session_step(Session* s, uint64_t k, std::string& err) {
     if (!s->slots && !s->resident && !s->graph_one[0]) { err = "this session steps only as part of a batch"; return FG_ERR_INVALID; }
     FG_CUDA(cudaSetDevice(s->gpu->device));
+    s->unchecked = true;
     uint64_t done = 0;
     if (s->resident) {
         while (done < k) {
@@ -2444,10 +2449,26 @@ int session_step(Session* s, uint64_t k, std::string& err) {
     return FG_OK;
 }
 
+int wait_error(int flag, std::string& err) {
+    err = "a bounded wait in the fused step ran out (code " + std::to_string(flag) + ")";
+    return FG_ERR_CUDA;
+}
+
+// The error word of the steps since the last look, once they have finished: the fields after a wait that
+// ran out are those of no step. The word stays set, so every later look reports it again.
+int session_check(Session* s, std::string& err) {
+    if (!s->unchecked) return FG_OK;
+    int flag = 0;
+    FG_CUDA(cudaMemcpy(&flag, s->error, sizeof(int), cudaMemcpyDeviceToHost));
+    if (flag) return wait_error(flag, err);
+    s->unchecked = false;
+    return FG_OK;
+}
+
 int session_sync(Session* s, std::string& err) {
     FG_CUDA(cudaSetDevice(s->gpu->device));
     FG_CUDA(cudaStreamSynchronize(s->stream));
-    return FG_OK;
+    return session_check(s, err);
 }
 
 // The buffers that hold the latest fields: after an odd number of fused steps, the second set.
@@ -2473,12 +2494,7 @@ int session_energy(Session* s, double* out, std::string& err) {
     FG_CUDA(cudaMemcpyAsync(part.data(), s->partial, ENERGY_BLOCKS * 8, cudaMemcpyDeviceToHost, s->stream));
     s->d2h_bytes += ENERGY_BLOCKS * 8;
     FG_CUDA(cudaStreamSynchronize(s->stream));
-    int flag = 0;
-    FG_CUDA(cudaMemcpy(&flag, s->error, sizeof(int), cudaMemcpyDeviceToHost));
-    if (flag) {
-        err = "a bounded wait in the fused step ran out (code " + std::to_string(flag) + ")";
-        return FG_ERR_CUDA;
-    }
+    if (const int rc = session_check(s, err)) return rc;
     double sum = 0.0;
     for (double v : part) sum += v;
     *out = sum;
@@ -2490,6 +2506,7 @@ uint64_t session_steps(const Session* s) { return s->steps; }
 int session_read(Session* s, const std::string& which, float* dst, uint64_t len, std::string& err) {
     FG_CUDA(cudaSetDevice(s->gpu->device));
     FG_CUDA(cudaStreamSynchronize(s->stream));
+    if (const int rc = session_check(s, err)) return rc;
     auto copy = [&](const float* src, uint64_t n) -> int {
         if (n > len) { err = "destination too small for " + which; return FG_ERR_INVALID; }
         if (n) FG_CUDA(cudaMemcpy(dst, src, n * 4, cudaMemcpyDeviceToHost));
@@ -2572,6 +2589,7 @@ int session_kernel_times(Session* s, uint64_t steps, std::vector<std::pair<std::
     std::vector<int> counts;
     // the two-step mode times double steps (one stream) and reports each kernel's time per step
     const uint64_t per = s->slots ? 2 : 1;
+    s->unchecked = true;
     if (const int rc = debye_states(*s, false, s->stream, err)) return rc;
     for (uint64_t q = 0; q < steps; q += per) {
         marks.clear();

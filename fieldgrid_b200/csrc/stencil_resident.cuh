@@ -62,6 +62,7 @@ struct ResArgs {
     unsigned* bar;                            // the grid barrier's arrivals, 0 at launch
     int* error;
     unsigned long long wait_ns;
+    unsigned late;                            // test knob, 0 in normal runs: arrivals every barrier waits for in vain
     FastDiv quads, rows;                      // 4-node groups per row; rows per plane
     unsigned last_row;                        // the grid's last row
     unsigned dq, drow, dj, di;                // a pass of the launch over its groups, as rows and groups; its rows as planes and rows
@@ -548,7 +549,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
     for (int q = threadIdx.x; q < a.ns; q += blockDim.x) own |= res_block_of(a, a.src[q].f, G, groups) == b;
     for (int q = threadIdx.x; q < a.ni; q += blockDim.x) own |= res_block_of(a, a.ind[q].f, G, groups) == b;
     own = __syncthreads_or(own);
-    unsigned target = 0;
+    unsigned target = a.late;
     for (int s = 0; s <= a.steps; ++s) {
         const unsigned n = n0 + unsigned(s);
         // ---- phase A: what reads E^n (E after step n - 1) ...
