@@ -12,8 +12,9 @@
 // cp.async), and a block's warps share the table of 32 directions. Its floor is the FP64 rate: 174,760
 // patches x 2664 directions are 11.2 G multiply-adds, 0.6 ms at 64 per SM and clock; the call takes
 // 2.0 ms where a block per direction took 13.4 with its copies.
-// Patches that do not come in lines (fewer than 8 per line on average) go through k_far_field, a block
-// per direction, which forms every phase.
+// Patches that do not come in lines (fewer than 8 per line on average), or whose lines hardly share their
+// sequences (FAR_SEQUENCES, FAR_PADDING), go through k_far_field, a block per direction, which forms every
+// phase.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -101,6 +102,13 @@ constexpr int FAR_LEN = 320;      // a line's patches at most (longer lines are 
 constexpr int FAR_WARPS = 8;
 constexpr int FAR_TILE = 8;       // patches of four lines a warp stages at a time
 constexpr int FAR_STAGE = 4 * FAR_TILE * 12;   // doubles
+// Sequences at most, each a block's table at least and sums of its own: a box has one or two per axis. Past
+// that, and where the slots of the blocks' passes (FAR_WARPS groups of four lines) would be more than
+// FAR_PADDING times the patches, k_far_field takes over: a pair costs it 6.7 times a filled slot (174,760
+// patches, 2664 directions: 13.4 ms against 2.0).
+constexpr size_t FAR_SEQUENCES = 4096;
+constexpr long long FAR_PADDING = 4;
+constexpr uint64_t FAR_PARTIAL = uint64_t(256) << 20;   // bytes of partial sums at a time, above 32 directions
 constexpr int FAR_SMEM = FAR_LEN * 32 * 16 + FAR_WARPS * 2 * FAR_STAGE * 8;
 
 __device__ __forceinline__ void cp16(void* dst, const void* src) {
@@ -311,10 +319,11 @@ int far_layout(Gpu* g, const double* pos, const double* area, const double* jm, 
         k_far_areas<<<148 * 8, 256>>>(D.jm, a, (long long)count);
         if (!check(cudaGetLastError(), "k_far_areas")) return FG_ERR_CUDA;
     }
+    std::vector<FarGroup> groups;
     if (D.lined) {
         // lines of one sequence, in their order, four to a group
         std::stable_sort(lines.begin(), lines.end(), [](const Line& a, const Line& b) { return a.seq < b.seq; });
-        std::vector<FarGroup> groups;
+        long long slots = 0;
         for (size_t i = 0; i < lines.size();) {
             size_t e = i;
             while (e < lines.size() && lines[e].seq == lines[i].seq) ++e;
@@ -331,8 +340,12 @@ int far_layout(Gpu* g, const double* pos, const double* area, const double* jm, 
             }
             r.g1 = int(groups.size());
             D.runs.push_back(r);
+            slots += (long long)((r.g1 - r.g0 + FAR_WARPS - 1) / FAR_WARPS) * FAR_WARPS * 4 * r.len;
             i = e;
         }
+        D.lined = D.runs.size() <= FAR_SEQUENCES && slots <= FAR_PADDING * (long long)count;
+    }
+    if (D.lined) {
         if (!check(cudaMalloc(&D.groups, groups.size() * sizeof(FarGroup)), "cudaMalloc") ||
             !check(cudaMalloc(&D.seqs, seqs.size() * 8), "cudaMalloc") ||
             !check(cudaMemcpy(D.groups, groups.data(), groups.size() * sizeof(FarGroup), cudaMemcpyHostToDevice), "cudaMemcpy") ||
@@ -388,10 +401,12 @@ int far_field_gpu(Gpu* g, std::vector<FarDevice*>& devices, const double* pos, c
             const int m = few ? 1 : FAR_WARPS * int(std::max<long long>(1, (per + pass / 2) / pass));
             for (int q = r.g0; q < r.g1; q += m) parts.push_back(FarPart{r.axis, r.len, r.seq, q, std::min(q + m, r.g1)});
         }
-        if (parts.size() > 65535) { err = "internal: too many far-field parts"; return FG_ERR_INVALID; }
     }
+    // directions at a time: no more partial sums than FAR_PARTIAL
+    const uint64_t step = parts.empty() ? MOST : std::min<uint64_t>(MOST, std::max<uint64_t>(32, FAR_PARTIAL / (96 * parts.size()) / 32 * 32));
+    const int ms = int(std::min<uint64_t>(n, step));
     const size_t pb = (parts.size() * sizeof(FarPart) + 255) & ~size_t(255);
-    const size_t bytes = pb + (size_t(9) * m0 + size_t(12) * parts.size() * m0) * 8 + 256;
+    const size_t bytes = pb + (size_t(9) + size_t(12) * parts.size()) * size_t(ms) * 8 + 256;
     if (D.work_bytes < bytes) {
         cudaFree(D.work);
         D.work = nullptr;
@@ -401,11 +416,11 @@ int far_field_gpu(Gpu* g, std::vector<FarDevice*>& devices, const double* pos, c
     }
     char* buf = D.work;
     double* d_dirs = reinterpret_cast<double*>(buf + pb);
-    double* d_out = d_dirs + 3 * size_t(m0);
-    double* d_part = d_out + 6 * size_t(m0);
+    double* d_out = d_dirs + 3 * size_t(ms);
+    double* d_part = d_out + 6 * size_t(ms);
     bool ok = parts.empty() || check(cudaMemcpyAsync(buf, parts.data(), parts.size() * sizeof(FarPart), cudaMemcpyHostToDevice, nullptr), "cudaMemcpy");
-    for (uint64_t first = 0; first < n && ok; first += MOST) {
-        const int m = int(std::min<uint64_t>(MOST, n - first));
+    for (uint64_t first = 0; first < n && ok; first += step) {
+        const int m = int(std::min<uint64_t>(step, n - first));
         ok = check(cudaMemcpyAsync(d_dirs, dirs + 3 * first, size_t(m) * 24, cudaMemcpyHostToDevice, nullptr), "cudaMemcpy");
         if (!ok) break;
         if (D.lined) {
