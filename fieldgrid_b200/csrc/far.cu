@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -271,7 +272,11 @@ void find_lines(const double* pos, int count, std::vector<Line>& lines, std::vec
 }  // namespace
 
 // What a Far keeps on its device: the currents times their areas, and the patches' lines (or, where
-// they form none, the positions). Laid out on the first call with the device's handle.
+// they form none, the positions). Laid out on the first call with the device's handle. All handles
+// together keep at most FAR_KEEP bytes: a call that ends above it gives its handle's back.
+constexpr long long FAR_KEEP = 1LL << 30;
+std::atomic<long long> far_kept{0};
+
 struct FarDevice {
     int device = 0;
     long long count = 0;
@@ -282,7 +287,9 @@ struct FarDevice {
     std::vector<Run> runs;
     char* work = nullptr;             // the calls' directions, parts and partial sums, grown as needed
     size_t work_bytes = 0;
+    long long bytes = 0, kept = 0;    // of the layout; what far_kept counts for this one
     ~FarDevice() {
+        far_kept -= kept;
         int prev = 0;
         const bool back = cudaGetDevice(&prev) == cudaSuccess;
         cudaSetDevice(device);
@@ -309,6 +316,7 @@ int far_layout(Gpu* g, const double* pos, const double* area, const double* jm, 
         find_lines(pos, int(count), lines, seqs);
         D.lined = lines.size() * 8 <= count;
     }
+    D.bytes = (long long)(13 * count * 8);
     // the currents, then their areas behind them for the products
     if (!check(cudaMalloc(&D.jm, std::max<size_t>(13 * count, 1) * 8), "cudaMalloc")) return FG_ERR_CUDA;
     if (count) {
@@ -346,6 +354,7 @@ int far_layout(Gpu* g, const double* pos, const double* area, const double* jm, 
         D.lined = D.runs.size() <= FAR_SEQUENCES && slots <= FAR_PADDING * (long long)count;
     }
     if (D.lined) {
+        D.bytes += (long long)(groups.size() * sizeof(FarGroup) + seqs.size() * 8);
         if (!check(cudaMalloc(&D.groups, groups.size() * sizeof(FarGroup)), "cudaMalloc") ||
             !check(cudaMalloc(&D.seqs, seqs.size() * 8), "cudaMalloc") ||
             !check(cudaMemcpy(D.groups, groups.data(), groups.size() * sizeof(FarGroup), cudaMemcpyHostToDevice), "cudaMemcpy") ||
@@ -353,6 +362,7 @@ int far_layout(Gpu* g, const double* pos, const double* area, const double* jm, 
             !check(cudaFuncSetAttribute(k_far_lines, cudaFuncAttributeMaxDynamicSharedMemorySize, FAR_SMEM), "cudaFuncSetAttribute"))
             return FG_ERR_CUDA;
     } else {
+        D.bytes += (long long)(3 * count * 8);
         if (!check(cudaMalloc(&D.pos, std::max<size_t>(3 * count, 1) * 8), "cudaMalloc") ||
             !check(cudaMemcpy(D.pos, pos, 3 * count * 8, cudaMemcpyHostToDevice), "cudaMemcpy"))
             return FG_ERR_CUDA;
@@ -435,6 +445,12 @@ int far_field_gpu(Gpu* g, std::vector<FarDevice*>& devices, const double* pos, c
              check(cudaMemcpyAsync(out + 6 * first, d_out, size_t(m) * 48, cudaMemcpyDeviceToHost, nullptr), "cudaMemcpy");
     }
     ok = check(cudaStreamSynchronize(nullptr), "far field") && ok;
+    const long long now = D.bytes + (long long)D.work_bytes, all = far_kept += now - D.kept;
+    D.kept = now;
+    if (all > FAR_KEEP) {
+        devices.erase(std::find(devices.begin(), devices.end(), &D));
+        delete &D;
+    }
     return ok ? FG_OK : FG_ERR_CUDA;
 }
 

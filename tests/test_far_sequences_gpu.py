@@ -43,3 +43,26 @@ def test_device_far_fields_equal_the_host_sums(gpu, sequences, share, length, di
         got = far.fields(d)
         assert np.isfinite(got).all()
         assert np.abs(got[some] - host).max() <= 1e-11 * np.abs(host).max()
+
+
+def test_the_handles_keep_a_bounded_share_of_the_device(gpu):
+    """A layout takes 104 bytes a patch and stays with its handle, of all handles together up to 1 GiB:
+    sixteen of 83 MB keep twelve, and the others are laid out by each call."""
+    import torch
+
+    pos = _lines(2, 40, 10000)
+    p = fdtd.Patches(pos, np.full(len(pos), 1e-6), np.zeros(0, np.uint32))
+    acc = np.random.RandomState(7).standard_normal((len(pos), 1, 12)).astype(np.float32)
+    d = np.array([[0.6, 0.0, 0.8], [0.0, 1.0, 0.0]])
+    free = lambda: torch.cuda.mem_get_info()[0]
+    first = fdtd.Far.load(p, acc, 1, 0, 9e9, gpu=gpu)
+    want = first.fields(d)
+    del first
+    start = free()
+    fars = [fdtd.Far.load(p, acc, 1, 0, 9e9, gpu=gpu) for _ in range(16)]
+    for _ in range(2):
+        for far in fars:
+            assert np.array_equal(far.fields(d), want)
+    assert start - free() < (1 << 30) + (96 << 20)
+    del far, fars
+    assert start - free() < 64 << 20
