@@ -2380,6 +2380,8 @@ int session_reset(Session* s, std::string& err) {
         FG_CUDA(cudaMemsetAsync(s->debye_old, 0, size_t(s->n_debye) * 4, st));
         FG_CUDA(cudaMemsetAsync(s->debye_state, 0, size_t(s->n_debye) * size_t(std::max(s->n_poles, 1)) * 4, st));
         s->rd_dense = false;   // the next resident step takes the list's
+        // the groups' other edges hold 0, or NaN once a field has left f32's range: no move rewrites them
+        if (s->rd_places) FG_CUDA(cudaMemsetAsync(s->rd_state, 0, s->rd_places * 48 * size_t(s->n_poles), st));
     }
     if (s->fold && s->nfold)
         FG_CUDA(cudaMemsetAsync(s->fstate, 0, size_t(s->nfold) * size_t(std::max(s->n_poles, 1)) * 4, st));
