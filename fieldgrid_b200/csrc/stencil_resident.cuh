@@ -316,8 +316,13 @@ __device__ __forceinline__ void res_update(const ResArgs& a, const ResNode* X, c
         if (sls >= 0) q_psi(S, ps, ds, q_bc(fs.b), q_bc(Y[j].c[F]), q_bc(fs.raw), z);
     } else {
         S = q_mul(ds, ld4(Z + (F ? 1 : 0) * np2 + k), z);
-        if (sls >= 0)
-            q_psi(S, ps, ds, ld4(Z + (F ? 4 : 6) * np2 + k), ld4(Z + (F ? 5 : 7) * np2 + k), ld4(Z + (F ? 3 : 2) * np2 + k), z);
+        if (sls >= 0) {
+            // the group's nodes outside the layer (b = 0) keep psi = 0 past f32's range too, where c d is NaN
+            const Quad b = ld4(Z + (F ? 4 : 6) * np2 + k);
+            const float2 o = make_float2(0.f, 0.f);
+            const Quad d{f2::pick(b.a.x != 0.f, b.a.y != 0.f, ds.a, o), f2::pick(b.b.x != 0.f, b.b.y != 0.f, ds.b, o)};
+            q_psi(S, ps, d, b, ld4(Z + (F ? 5 : 7) * np2 + k), ld4(Z + (F ? 3 : 2) * np2 + k), z);
+        }
     }
     if (sls >= 0) st4(psi_out + os, ps);
     const Quad t = C == 1 ? S - R : R - S;
