@@ -592,6 +592,7 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
     int cid = 1;
     for (const HostSim* h : sims) cid = std::max(cid, h->classes.size() <= 256 ? 1 : (h->classes.size() <= 65536 ? 2 : 4));
     B->cid_bytes = cid;
+    bool debye_groups = true;
     for (size_t b = 0; b < sims.size(); ++b) {
         const HostSim& h = *sims[b];
         if (!h.wires.empty() || !h.sheets.empty()) { err = "grid " + std::to_string(b) + ": a batch takes no thin wires or resistive sheets"; return FG_ERR_INVALID; }
@@ -600,9 +601,17 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
         rs.fused = true;
         rs.graphs = false;
         rs.cid_bytes = cid;
+        rs.debye_groups = debye_groups;
         rs.tma_seg = 64;   // the other grids fill the GPU: long segments, few halo planes
         Session* s = nullptr;
         const int rc = session_new(gpu, h, rs, &s, err);
+        if (rc == FG_ERR_TOO_LARGE && debye_groups) {   // once more, every grid without the resident steps' extra room
+            debye_groups = false;
+            for (Session* x : B->s) session_free(x);
+            B->s.clear();
+            b = size_t(-1);
+            continue;
+        }
         if (rc) { err = "grid " + std::to_string(b) + ": " + err; return rc; }
         B->s.push_back(s);
     }

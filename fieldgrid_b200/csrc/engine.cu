@@ -1844,13 +1844,16 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     need += carve_size(std::max<size_t>(nd, 1) * 8);
     need += carve_size(std::max<size_t>(nd, 1) * 4) * 3;
     need += carve_size(std::max<size_t>(nd * sim.poles.size(), 1) * 4);
-    // the Debye edges by groups, where the grid may step resident (32-bit offsets)
+    // the Debye edges by groups, where the grid may step resident (32-bit offsets) and the device has the
+    // room: they come on top of the list, and a grid that fits without them is not refused
     const size_t rgroups = n0 * n1 * ((n2 + 3) / 4);
-    s->rd_places = s->k_quads && nd > 0 && nd < (size_t(1) << 31) ? std::min(nd, rgroups) : 0;
+    size_t rd_need = 0;
+    s->rd_places = rs.debye_groups && s->k_quads && resident_allowed(*s) && nd > 0 && nd < (size_t(1) << 31) ? std::min(nd, rgroups) : 0;
     if (s->rd_places * 12 * std::max<size_t>(sim.poles.size(), 1) >= (size_t(1) << 32)) s->rd_places = 0;
     if (s->rd_places) {
         FG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, s->rd_tmp_bytes, (const int*)nullptr, (int*)nullptr, int(rgroups), nullptr));
-        need += carve_size(rgroups * 4) * 2 + carve_size(s->rd_places * 48) * (1 + sim.poles.size()) + carve_size(s->rd_tmp_bytes);
+        rd_need = carve_size(rgroups * 4) * 2 + carve_size(s->rd_places * 48) * (1 + sim.poles.size()) + carve_size(s->rd_tmp_bytes);
+        need += rd_need;
     }
     // the host records, set-up only: packed to 8 bytes while staged where the device nodes allow
     const bool pack_debye = nnp < (size_t(1) << 30);
@@ -1876,6 +1879,10 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     if (!gp->spare) {
         size_t free_b = 0, total_b = 0;
         FG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        if (need + (size_t(256) << 20) > free_b) {
+            need -= rd_need;
+            s->rd_places = 0;
+        }
         if (need + (size_t(256) << 20) > free_b) {
             err = std::to_string(sim.cells()) + " cells is more than this GPU can hold";
             return FG_ERR_TOO_LARGE;
