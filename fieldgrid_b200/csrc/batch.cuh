@@ -670,6 +670,8 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
     if (!tune && fixed.tile == BATCH_RESIDENT) {
         share = std::min(std::max(fixed.blocks_per_sm, 1), 4);
         if ((rc = batch_plan_resident(*B, share, err))) return rc;
+        while (!B->resident_ok && share > 1)   // as many as fit on an SM
+            if ((rc = batch_plan_resident(*B, --share, err))) return rc;
         if (B->resident_ok) {
             best = BatchShape{BATCH_BRANCHES, 0, 0};
         } else {   // a grid that cannot: the merged launches, as any number past theirs always chose

@@ -890,6 +890,7 @@ int plan_resident(Session& s, int share, std::string& err) {
         return FG_OK;
     });
     if (rc) return rc;
+    if (!s.res_cluster && per < share) return FG_OK;   // a long axis's factors: less room than the threads leave
     if (per < 1) return FG_OK;
     if (const int rb = rd_build(s, err)) return rb;
     s.resident = true;
