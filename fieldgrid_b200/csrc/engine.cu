@@ -846,7 +846,8 @@ int debye_states(Session& s, bool dense, cudaStream_t st, std::string& err) {
 }
 
 // Whether a session's steps may run resident: not where a pipeline is asked for by name
-// (FIELDGRID_RESIDENT=0 rules it out), nor with thin wires or resistive sheets.
+// (FIELDGRID_RESIDENT=0 rules it out; "grid" keeps small grids off the cluster launch), nor with thin wires
+// or resistive sheets.
 bool resident_allowed(const Session& s) {
     const char* rv = std::getenv("FIELDGRID_RESIDENT");
     const char* nv = std::getenv("FIELDGRID_NO_TMA");
@@ -859,6 +860,26 @@ int with_adj_resident(int cid_bytes, bool cluster, F&& f) {
     if (cid_bytes == 1) return cluster ? f(k_adj_resident<uint8_t, true>) : f(k_adj_resident<uint8_t, false>);
     if (cid_bytes == 2) return cluster ? f(k_adj_resident<uint16_t, true>) : f(k_adj_resident<uint16_t, false>);
     return cluster ? f(k_adj_resident<uint32_t, true>) : f(k_adj_resident<uint32_t, false>);
+}
+
+// A resident launch: one cluster, or a cooperative launch.
+cudaLaunchConfig_t res_config(const Session& s, size_t smem, cudaStream_t st, cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(s.res_blocks));
+    cfg.blockDim = dim3(unsigned(3 * s.res_groups));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    if (s.res_cluster) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = unsigned(s.res_blocks);
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
 }
 
 // Whether a session's steps run resident, and its launch shape, with room on each SM for the blocks of
@@ -877,21 +898,38 @@ int plan_resident(Session& s, int share, std::string& err) {
         const long long even = ((total + blocks * passes - 1) / (blocks * passes) + 31) / 32 * 32;   // passes of one size
         return int(std::min(most, std::max<long long>(32, passes <= 4 ? even : most)));
     };
-    s.res_cluster = total <= RES_CLUSTER_GROUPS && !s.stall_barrier;   // the cluster's own barrier cannot run out
-    const int most = s.res_cluster ? RES_CLUSTER : sms;
-    s.res_groups = groups_of(most);
-    s.res_blocks = s.res_cluster ? RES_CLUSTER : int(std::min<long long>(sms, (total + s.res_groups - 1) / s.res_groups));
     const size_t smem = res_smem(g);
-    const int rc = with_resident(s, [&](auto kern) -> int {
-        FG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(size_t(res_pad(RES_MAX_AXES + 9)) * 48)));
-        if (s.res_cluster) FG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        FG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 3 * s.res_groups, smem));
-        return FG_OK;
-    });
-    if (rc) return rc;
-    if (!s.res_cluster && per < share) return FG_OK;   // a long axis's factors: less room than the threads leave
-    if (per < 1) return FG_OK;
+    // the launch's shape, and how many of its blocks an SM takes (of a cluster: how many the device does)
+    auto shape = [&](bool cluster) -> int {
+        s.res_cluster = cluster;
+        s.res_groups = groups_of(cluster ? RES_CLUSTER : sms);
+        s.res_blocks = cluster ? RES_CLUSTER : int(std::min<long long>(sms, (total + s.res_groups - 1) / s.res_groups));
+        return with_resident(s, [&](auto kern) -> int {
+            FG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         int(size_t(res_pad(RES_MAX_AXES + 9)) * 48)));
+            if (!cluster) {
+                FG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 3 * s.res_groups, smem));
+                return FG_OK;
+            }
+            FG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            cudaLaunchAttribute at[1];
+            const cudaLaunchConfig_t cfg = res_config(s, smem, nullptr, at);
+            if (cudaOccupancyMaxActiveClusters(&per, kern, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                per = 0;
+            }
+            return FG_OK;
+        });
+    };
+    // the cluster's own barrier cannot run out; a device or a partition without room for 16 blocks of one
+    // cluster takes the grid's
+    int rc = FG_OK;
+    const char* rv = std::getenv("FIELDGRID_RESIDENT");
+    if (total <= RES_CLUSTER_GROUPS && !s.stall_barrier && !(rv && std::strcmp(rv, "grid") == 0) && (rc = shape(true))) return rc;
+    if (per < 1) {
+        if ((rc = shape(false))) return rc;
+        if (per < share) return FG_OK;   // a long axis's factors: less room than the threads leave
+    }
     if (const int rb = rd_build(s, err)) return rb;
     s.resident = true;
     return FG_OK;
@@ -929,26 +967,12 @@ void resident_shape(const Session& s, ResArgs& a) {
     a.n_debye = s.n_debye;
 }
 
-// Launches a resident kernel on `st` with every block resident: one cluster, or a cooperative launch.
+// Launches a resident kernel on `st` with every block resident.
 template <typename K, typename A>
 int launch_res(const Session& s, K kern, const A& a, size_t smem, cudaStream_t st, std::string& err) {
     if (!s.res_cluster) FG_CUDA(cudaMemsetAsync(s.res_bar, 0, sizeof(unsigned), st));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(unsigned(s.res_blocks));
-    cfg.blockDim = dim3(unsigned(3 * s.res_groups));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
     cudaLaunchAttribute at[1];
-    if (s.res_cluster) {
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = unsigned(s.res_blocks);
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    } else {
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-    }
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    const cudaLaunchConfig_t cfg = res_config(s, smem, st, at);
     FG_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
     return FG_OK;
 }
