@@ -9,7 +9,7 @@ from fieldgrid_b200 import workloads as W
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("cells", [12, 24])
+@pytest.mark.parametrize("cells", [14, 22])
 def test_small_grids_step_by_either_barrier(gpu, monkeypatch, cells):
     sc = W.spheres(cells, pml=4, count=4, rmin=2, rmax=5, steps=40, fused=True)
     sim = fdtd.Sim.try_new(*sc.args())
