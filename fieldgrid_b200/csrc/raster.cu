@@ -407,14 +407,9 @@ size_t partition(const std::vector<double>& line, double v, bool or_equal) {
         }                                                                                          \
     } while (0)
 
-// fill (raster.rs:24-104) on the device: inside / thin get 1 at the filled samples, indexed in the
-// space of dimensions dims (order 0: (i m1 + j) m2 + k, 1: i + (j + k m1) m0; every sample index
-// is below its dimension); thin is then cleared where inside is set.
-int raster_fill(Gpu* gpu, const double* tris, uint64_t ntri, const std::vector<double>* samples, const size_t* dims,
+static int fill_masks(Gpu* gpu, const double* tris, uint64_t ntri, const std::vector<double>* samples, const size_t* dims,
                 int order, uint8_t* inside, uint8_t* thin, std::string& err) {
     using namespace raster;
-    for (int a = 0; a < 3; ++a)
-        if (samples[a].size() > dims[a]) { err = "a sample line is longer than its index dimension"; return FG_ERR_INVALID; }
     const size_t total = dims[0] * dims[1] * dims[2];
     auto nothing = [&] {
         std::memset(inside, 0, total);
@@ -422,7 +417,7 @@ int raster_fill(Gpu* gpu, const double* tris, uint64_t ntri, const std::vector<d
         return FG_OK;
     };
     if (ntri == 0 || total == 0) return nothing();
-    if (ntri >= (uint64_t(1) << 31)) { nothing(); err = "too many triangles"; return FG_ERR_INVALID; }
+    if (ntri >= (uint64_t(1) << 31)) { err = "too many triangles"; return FG_ERR_INVALID; }
     RS_CUDA(cudaSetDevice(gpu->device));
     double low[3], high[3];   // the mesh's box
     for (int a = 0; a < 3; ++a) { low[a] = INFINITY; high[a] = -INFINITY; }
@@ -578,6 +573,22 @@ int raster_fill(Gpu* gpu, const double* tris, uint64_t ntri, const std::vector<d
         return FG_ERR_INVALID;
     }
     return FG_OK;
+}
+
+// fill (raster.rs:24-104) on the device: inside / thin get 1 at the filled samples, indexed in the
+// space of dimensions dims (order 0: (i m1 + j) m2 + k, 1: i + (j + k m1) m0; every sample index
+// is below its dimension); thin is then cleared where inside is set. A fill that fails leaves both clear.
+int raster_fill(Gpu* gpu, const double* tris, uint64_t ntri, const std::vector<double>* samples, const size_t* dims,
+                int order, uint8_t* inside, uint8_t* thin, std::string& err) {
+    for (int a = 0; a < 3; ++a)
+        if (samples[a].size() > dims[a]) { err = "a sample line is longer than its index dimension"; return FG_ERR_INVALID; }
+    const int rc = fill_masks(gpu, tris, ntri, samples, dims, order, inside, thin, err);
+    if (rc) {
+        std::memset(inside, 0, dims[0] * dims[1] * dims[2]);
+        std::memset(thin, 0, dims[0] * dims[1] * dims[2]);
+        cudaGetLastError();   // a failed allocation is not the next call's error
+    }
+    return rc;
 }
 
 int raster_sheet_edges(Gpu* gpu, const double* tris, uint64_t ntri, const std::vector<double>* lines, uint8_t* mask,
