@@ -66,6 +66,8 @@ def _declare(L):
         "fg_record_h": (P(C.c_float), [vp, P(u64)]),
         "fg_record_transfer": (None, [vp, P(u64), P(u64)]),
         "fg_record_free": (None, [vp]),
+        "fg_record_take": (vp, [vp, P(C.c_float)]),
+        "fg_array_free": (None, [vp]),
         "fg_session_kernel_times": (C.c_int, [vp, u64, cp, P(dbl), u64, P(u64)]),
         "fg_session_new": (C.c_int, [vp, vp, u64, P(A.fg_pulse), P(A.fg_extras), P(vp), cp, sz]),
         "fg_session_step": (C.c_int, [vp, u64]),

@@ -9,6 +9,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <sys/mman.h>
@@ -110,6 +111,10 @@ struct HostArray {
     const float* data() const { return p; }
     size_t size() const { return n; }
     bool empty() const { return n == 0; }
+    float* release() {   // the caller frees it
+        n = 0;
+        return std::exchange(p, nullptr);
+    }
     HostArray() = default;
     HostArray(const HostArray&) = delete;
     HostArray& operator=(const HostArray&) = delete;
@@ -381,6 +386,13 @@ void fg_record_transfer(const fg_record* r, uint64_t* h2d, uint64_t* d2h) {
     if (d2h) *d2h = r ? r->d2h : 0;
 }
 void fg_record_free(fg_record* r) { delete r; }
+float* fg_record_take(fg_record* r, const float* array) {
+    if (!r || !array) return nullptr;
+    for (HostArray* a : {&r->series, &r->plane, &r->ntff, &r->e, &r->h})
+        if (a->p == array) return a->release();
+    return nullptr;
+}
+void fg_array_free(float* array) { std::free(array); }
 
 int fg_session_kernel_times(fg_session* s, uint64_t steps, char* names, double* ms, uint64_t cap, uint64_t* count) {
     if (!s || !count) return FG_ERR_INVALID;

@@ -329,28 +329,28 @@ class Record:
     d2h: int = 0
 
 
-class _RecordHandle:
-    """An engine record; freed with the last array that views it."""
+class _Owned:
+    """An array taken from an engine record; freed with the numpy array over it."""
 
-    def __init__(self, handle):
-        self.handle = handle
+    def __init__(self, address):
+        self.address = address
 
     def __del__(self):
         try:
-            lib().fg_record_free(self.handle)
+            lib().fg_array_free(self.address)
         except Exception:
             pass
 
 
-def _array(owner: _RecordHandle, ptr, n) -> np.ndarray:
-    """A record's array: a copy of a small one, else a view of the record's own memory (which it keeps
-    alive; nothing else reads or writes it)."""
+def _array(record, ptr, n) -> np.ndarray:
+    """A record's array: a copy of a small one, else the array itself, taken from the record."""
     if not ptr or n == 0:
         return np.zeros(0, np.float32)
     if n < 1 << 18:
         return np.ctypeslib.as_array(ptr, shape=(n,)).copy()
-    buf = (C.c_float * n).from_address(C.addressof(ptr.contents))
-    buf._owner = owner
+    own = _Owned(lib().fg_record_take(record, ptr))
+    buf = (C.c_float * n).from_address(own.address)
+    buf._owner = own
     return np.frombuffer(buf, np.float32)
 
 
@@ -378,23 +378,25 @@ def run(g, sim: Sim, driven: int, pulse: Pulse, extras: Extras,
     if exc:
         raise exc[0]
     _check(code, err)
-    own = _RecordHandle(out)
-    n = C.c_uint64()
-    rec = Record(
-        steps=int(L.fg_record_steps(out)),
-        ports=int(L.fg_record_ports(out)),
-        series=_array(own, L.fg_record_series(out, C.byref(n)), n.value),
-        decay_db=float(L.fg_record_decay_db(out)),
-        plane=_array(own, L.fg_record_plane(out, C.byref(n)), n.value),
-        ntff=_array(own, L.fg_record_ntff(out, C.byref(n)), n.value),
-    )
-    if keep_fields:
-        rec.e = _array(own, L.fg_record_e(out, C.byref(n)), n.value)
-        rec.h = _array(own, L.fg_record_h(out, C.byref(n)), n.value)
-    a, b = C.c_uint64(), C.c_uint64()
-    L.fg_record_transfer(out, C.byref(a), C.byref(b))
-    rec.h2d, rec.d2h = int(a.value), int(b.value)
-    return rec
+    try:
+        n = C.c_uint64()
+        rec = Record(
+            steps=int(L.fg_record_steps(out)),
+            ports=int(L.fg_record_ports(out)),
+            series=_array(out, L.fg_record_series(out, C.byref(n)), n.value),
+            decay_db=float(L.fg_record_decay_db(out)),
+            plane=_array(out, L.fg_record_plane(out, C.byref(n)), n.value),
+            ntff=_array(out, L.fg_record_ntff(out, C.byref(n)), n.value),
+        )
+        if keep_fields:
+            rec.e = _array(out, L.fg_record_e(out, C.byref(n)), n.value)
+            rec.h = _array(out, L.fg_record_h(out, C.byref(n)), n.value)
+        a, b = C.c_uint64(), C.c_uint64()
+        L.fg_record_transfer(out, C.byref(a), C.byref(b))
+        rec.h2d, rec.d2h = int(a.value), int(b.value)
+        return rec
+    finally:
+        L.fg_record_free(out)
 
 
 run_blocking = run

@@ -191,6 +191,10 @@ const float* fg_record_h(const fg_record* r, uint64_t* len);
  * device->host (energy partials, series, plane, ntff, fields). */
 void fg_record_transfer(const fg_record* r, uint64_t* h2d, uint64_t* d2h);
 void fg_record_free(fg_record* r);
+/* Hands one of the record's arrays (a pointer that a getter above returned) over to the caller, who frees
+ * it with fg_array_free; the record no longer has it. NULL: not an array of this record. */
+float* fg_record_take(fg_record* r, const float* array);
+void fg_array_free(float* array);
 
 /* ---- device-resident session: the buffers of one run, stepped explicitly ------------------
  * fg_run is fg_session_new + chunks of fg_session_step + energy checks + reads. The session
