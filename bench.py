@@ -340,11 +340,14 @@ def run_antenna(args):
     clocks = sampler.stop()
     ms = max_over_ranks(ev0.elapsed_time(ev1), world)
     kt = s.kernel_times(kt_steps)
-    launches = s.launches_per_step
+    launches = s.launches(K)
     variant = s.variant
     s.close()
     field_parts = [k for k in ("fused_step", "shell_h", "shell_e", "update_h", "update_e") if k in kt]
     dom_ms = sum(kt[k] for k in field_parts)
+    dom_name = "field_update"
+    if "resident" in variant:   # the whole step is one kernel's; kernel_ms are the one-step kernels'
+        field_parts, dom_name, dom_ms = ["k_resident"], "k_resident", ms / K
     total_kt = sum(kt.values())
     peak, peak_src = measured_peaks()
     achieved = BYTES_PER_NODE * nn / (dom_ms / 1e3) / 1e9
@@ -374,13 +377,13 @@ def run_antenna(args):
         "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": sc.name + ", NTFF box at 8/10/12 GHz", "nodes": nn, "pml": sc.info["pml"],
                    "patches": int(len(pt.area)), "freqs": list(sc.extras.freqs), "variant": variant,
-                   "launches_per_step": launches},
+                   "launches_per_step": launches / K},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "kernel": "field_update", "kernels": field_parts, "kernel_ms": dom_ms, "peak_source": peak_src},
+                     "kernel": dom_name, "kernels": field_parts, "kernel_ms": dom_ms, "peak_source": peak_src},
         "kernel_ms": {k: round(v, 5) for k, v in kt.items()},
         "kernel_share": {k: round(v / total_kt, 4) for k, v in kt.items()},
         "ntff_share": round(kt.get("ntff", 0.0) / total_kt, 4),
-        "gpu_launches": launches * K,
+        "gpu_launches": launches,
         "clocks": clocks,
         "e2e": {"value": job_rate(nn, K, world, t_e2e * 1e3), "unit": "Mcell/s", "h2d_bytes_per_step": rec.h2d / K,
                 "d2h_bytes_per_step": rec.d2h / K,
@@ -590,7 +593,7 @@ def main():
 
     # per-kernel device times of the same step (events between eager launches)
     kt = s.kernel_times(kt_steps)
-    launches = s.launches_per_step
+    launches = s.launches(K)
     energy = s.energy()
     variant = s.variant
     classes = sim.coef_classes()
@@ -603,6 +606,8 @@ def main():
     field_parts = [k for k in ("two_step", "edge_step", "fused_step", "shell_h", "shell_e", "update_h", "update_e")
                    if k in kt]
     dom_name, dom_ms = "field_update", sum(kt[k] for k in field_parts)
+    if "resident" in variant:   # the whole step is one kernel's; kernel_ms are the one-step kernels'
+        field_parts, dom_name, dom_ms = ["k_resident"], "k_resident", ms_max / K
     peak, peak_src = measured_peaks()
     achieved = BYTES_PER_NODE * nn / (dom_ms / 1e3) / 1e9
     total_kt = sum(kt.values())
@@ -655,7 +660,7 @@ def main():
                        "spheres": sc.info.get("spheres"), "parallelism": f"replicas x{world}",
                        "l2": "inputs larger than L2 (6.5 GB of fields per buffer set)",
                        "variant": variant, "coef_classes": classes, "debye_edges": debye_edges,
-                       "launches_per_step": launches, "setup_s": round(t_setup, 2)},
+                       "launches_per_step": launches / K, "setup_s": round(t_setup, 2)},
             "hbm_fraction_of_algorithmic": BYTES_PER_NODE * value * 1e6 / world / 1e9 / peak,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic_for(dom_name, sc.name), "kernel": dom_name,
@@ -663,7 +668,7 @@ def main():
                          "bytes_per_launch": BYTES_PER_NODE * nn, "kernel_ms": dom_ms, "peak_source": peak_src},
             "kernel_ms": {k: round(v, 5) for k, v in kt.items()},
             "kernel_share": {k: round(v / total_kt, 4) for k, v in kt.items()},
-            "gpu_launches": launches * K,
+            "gpu_launches": launches,
             "clocks": clocks,
             "e2e": e2e,
             "cpu_baseline": cpu,

@@ -77,6 +77,7 @@ def _declare(L):
         "fg_session_read": (C.c_int, [vp, cp, P(C.c_float), u64]),
         "fg_session_stream": (vp, [vp]),
         "fg_session_launches_per_step": (u64, [vp]),
+        "fg_session_launches": (u64, [vp, u64]),
         "fg_session_device_bytes": (u64, [vp]),
         "fg_session_variant": (cp, [vp]),
         "fg_session_free": (None, [vp]),

@@ -283,6 +283,7 @@ int fg_session_read(fg_session* s, const char* which, float* dst, uint64_t len) 
 }
 
 void* fg_session_stream(fg_session* s) { return s ? session_stream(s->s) : nullptr; }
+uint64_t fg_session_launches(const fg_session* s, uint64_t steps) { return s ? session_launches(s->s, steps) : 0; }
 uint64_t fg_session_launches_per_step(const fg_session* s) { return s ? session_launches_per_step(s->s) : 0; }
 uint64_t fg_session_device_bytes(const fg_session* s) { return s ? session_device_bytes(s->s) : 0; }
 const char* fg_session_variant(const fg_session* s) { return s ? session_variant(s->s) : ""; }

@@ -2587,6 +2587,11 @@ int session_read(Session* s, const std::string& which, float* dst, uint64_t len,
 
 void* session_stream(Session* s) { return s->stream; }
 uint64_t session_launches_per_step(const Session* s) { return s->launches; }
+uint64_t session_launches(const Session* s, uint64_t steps) {
+    if (!s->resident) return s->launches * steps;
+    const uint64_t most = resident_steps(*s);
+    return (steps + most - 1) / most;
+}
 uint64_t session_device_bytes(const Session* s) { return s->arena_bytes; }
 const char* session_variant(const Session* s) { return s->variant.c_str(); }
 uint64_t session_ports(const Session* s) { return uint64_t(s->sc.ports); }
@@ -2611,7 +2616,8 @@ void session_profile(Session* s) {
         std::fprintf(stderr, "fdtd kernel %s: %.1f us over 20 launches\n", name.c_str(), 1e3 * ms);
         step += ms;
     }
-    std::fprintf(stderr, "fdtd kernel time per step: %.1f us (%s)\n", 1e3 * step, s->variant.c_str());
+    std::fprintf(stderr, "fdtd kernel time per step: %.1f us (%s)%s\n", 1e3 * step, s->variant.c_str(),
+                 s->resident ? "; of the one-step kernels, which the run's resident steps do not launch" : "");
 }
 
 // Launches `steps` steps one kernel at a time with an event before each launch.

@@ -77,6 +77,7 @@ uint64_t session_steps(const Session* s);
 int session_read(Session* s, const std::string& which, float* dst, uint64_t len, std::string& err);
 void* session_stream(Session* s);
 uint64_t session_launches_per_step(const Session* s);
+uint64_t session_launches(const Session* s, uint64_t steps);
 uint64_t session_device_bytes(const Session* s);
 const char* session_variant(const Session* s);
 uint64_t session_ports(const Session* s);

@@ -446,7 +446,8 @@ class Session:
 
     def kernel_times(self, steps: int) -> dict:
         """Mean device ms per launch of each kernel of a step, over `steps` steps launched one
-        kernel at a time (the steps count as steps of the run)."""
+        kernel at a time (the steps count as steps of the run). Of a session that steps resident:
+        of the one-step kernels that would step it otherwise."""
         cap = 32
         names = C.create_string_buffer(64 * cap)
         ms = (C.c_double * cap)()
@@ -464,8 +465,13 @@ class Session:
     def stream(self) -> int:
         return int(lib().fg_session_stream(self._h) or 0)
 
+    def launches(self, steps: int) -> int:
+        """Kernel launches that step(steps) enqueues."""
+        return int(lib().fg_session_launches(self._h, steps))
+
     @property
     def launches_per_step(self) -> int:
+        """Kernel launches of a step by the one-step kernels (see kernel_times)."""
         return int(lib().fg_session_launches_per_step(self._h))
 
     @property

@@ -201,9 +201,10 @@ void fg_array_free(float* array);
  * keeps every buffer in HBM between calls, so a caller can time the step loop alone. */
 int fg_session_new(fg_gpu* g, const fg_sim* sim, uint64_t driven, const fg_pulse* pulse,
                    const fg_extras* extras, fg_session** out, char* err, size_t errlen);
-/* Enqueue k time steps on the session's stream (CUDA-graph replays); does not wait. */
+/* Enqueue k time steps on the session's stream (CUDA-graph replays, or resident launches of many steps);
+ * does not wait. */
 int fg_session_step(fg_session* s, uint64_t k);
-/* Wait for the session's stream. */
+/* Wait for the session's stream; FG_ERR_CUDA if a bounded wait of a step ran out (as energy and read). */
 int fg_session_sync(fg_session* s);
 /* Sum of E^2 + (376.73 H)^2 over the current fields (cpu.rs:417-421), waits. */
 int fg_session_energy(fg_session* s, double* out);
@@ -214,14 +215,18 @@ uint64_t fg_session_steps(const fg_session* s);
 int fg_session_read(fg_session* s, const char* which, float* dst, uint64_t len);
 /* The CUDA stream the session launches on (a cudaStream_t), for event timing. */
 void* fg_session_stream(fg_session* s);
-/* Kernel launches one time step enqueues (for launch accounting). */
+/* Kernel launches fg_session_step enqueues for `steps` steps (for launch accounting). */
+uint64_t fg_session_launches(const fg_session* s, uint64_t steps);
+/* Kernel launches of one time step by the one-step kernels, those of fg_session_kernel_times (a session
+ * that steps resident launches one kernel for many steps instead). */
 uint64_t fg_session_launches_per_step(const fg_session* s);
 /* Device bytes the session holds. */
 uint64_t fg_session_device_bytes(const fg_session* s);
 /* Per-kernel device times of `steps` steps launched one kernel at a time with CUDA events
  * between the launches (the report of run.rs:153-176). Fills up to `cap` entries of names
  * (each up to 63 chars + NUL, 64 bytes per entry) and mean ms per launch; *count = kernels per
- * step. The steps count as steps of the run. */
+ * step. The steps count as steps of the run. Of a session that steps resident: of the one-step kernels
+ * that would step it otherwise. */
 int fg_session_kernel_times(fg_session* s, uint64_t steps, char* names, double* ms, uint64_t cap, uint64_t* count);
 /* Name of the stencil kernel variant in use and its tile shape. */
 const char* fg_session_variant(const fg_session* s);
