@@ -16,9 +16,9 @@
 // launches above: seven launches per step for the whole batch, with each grid's arithmetic that of
 // its own TMA step.
 //
-// Resident mode (tile 6): where every grid's state fits the L2, each grid steps on its own, many steps in
-// one resident launch (stencil_resident.cuh) before the next grid's: its fields stay in the L2 over those
-// steps, where the other modes carry every grid's fields through HBM each step. blocks_per_sm launches
+// Resident mode (tile 6): where every grid can (up to 23 M nodes), each grid steps on its own, many steps in
+// one resident launch (stencil_resident.cuh) before the next grid's: up to about 4 M nodes its fields stay in
+// the L2 over those steps, where the other modes carry every grid's fields through HBM each step. blocks_per_sm launches
 // run side by side, so that one grid's barriers hide behind another's work. Calls of few steps go
 // through the graphs of the fastest other mode.
 //

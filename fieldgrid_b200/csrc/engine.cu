@@ -136,12 +136,14 @@ int staged_upload(Gpu* g, void* dst, const void* src, size_t bytes, void* stream
 // Steps of one resident launch at most, and nodes times steps (a bound on the time one kernel holds the GPU).
 constexpr uint64_t RES_MAX_STEPS = 1024;
 constexpr long long RES_MAX_WORK = 1LL << 32;
-// Nodes of a grid stepped resident at most. In the fused mode the TMA march's graphs take over where they
-// move fewer bytes at the HBM rate; the separate kernels are slower at every size (32-bit field offsets
-// bound it). Measured us per step, resident / march / separate: 65^3 9 / 35 / 21; 121^3 with Debye
-// spheres 30 / 64 / 57; 145^3 56 / 97 / 130; 201^3 129 / 175 / 320; 261^3 265 / 335 / 668;
-// 299^3 490 / 465.
-constexpr long long RES_MAX_FUSED = 22LL << 20, RES_MAX_SEPARATE = 1LL << 28;
+// Nodes of a grid stepped resident at most in the fused mode, where the TMA march's graphs take over: they
+// move fewer bytes at the HBM rate. The separate kernels are slower at every size; what bounds those grids
+// is the axes' factors (RES_MAX_AXES nodes of the three together, so 2^27 nodes) and 32-bit field offsets.
+// Measured us per step, resident / march / separate: 65^3 9 / 35 / 21; 121^3 with Debye spheres 30 / 64 /
+// 57; 145^3 56 / 97 / 130; 201^3 127 / 175 / 320; 261^3 265 / 335 / 668; 299^3 490 / 465; resident /
+// separate: 301^3 386 / 904; 401^3 894 / 2118; 501^3 1817 / 3861; 901x501x131 1014 / 2567; 131x501x901
+// 821 / 1910.
+constexpr long long RES_MAX_FUSED = 22LL << 20;
 // 4-node groups of a grid stepped by one cluster at most: its barrier is shorter than a grid-wide one,
 // but 16 SMs share the work (29x19x14: 4.1 us a step against 5.2; 25^3: 6.5 against 6.5).
 constexpr long long RES_CLUSTER_GROUPS = 4096;
@@ -1637,7 +1639,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     // the k axis as the device keeps it: on grids of a size that steps resident, with its layer's slots
     // numbered by 4-node groups where that is possible
     std::vector<AxisNode> kax_node = sim.ax[2].node;
-    s->k_quads = (long long)nn <= (s->fused ? RES_MAX_FUSED : RES_MAX_SEPARATE) && 3 * g.cs < (1LL << 32) && n0 + n1 + n2 <= size_t(RES_MAX_AXES) && res_k_slots(kax_node, sim.pml, g.pw);
+    s->k_quads = (!s->fused || (long long)nn <= RES_MAX_FUSED) && 3 * g.cs < (1LL << 32) && n0 + n1 + n2 <= size_t(RES_MAX_AXES) && res_k_slots(kax_node, sim.pml, g.pw);
     long long psi_total = 0, psi_hbase = 0;
     for (int e = 0; e < 2; ++e) {
         if (e == 1) psi_hbase = psi_total;

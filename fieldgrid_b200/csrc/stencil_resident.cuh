@@ -1,12 +1,15 @@
-// Many time steps in one launch, for grids whose state stays in L2: a cooperative kernel with the
-// whole grid's blocks resident steps E and H in place, half a step at a time, with a grid-wide
-// barrier between the halves (two per step; a third where a design history follows the E half).
+// Many time steps in one launch: a cooperative kernel with the whole grid's blocks resident steps E and H
+// in place, half a step at a time, with a grid-wide barrier between the halves (two per step; a third where
+// a design history follows the E half). For grids of up to 23 M nodes by the fused step, and every separate
+// run whose axes' factors fit shared memory (engine.cu, RES_MAX_FUSED and RES_MAX_AXES).
 //
 // The march kernels move each field once per step through HBM, but a march is a chain of planes: a
 // small grid leaves most SMs idle behind it (65^3: 42 blocks, 33 us a step). In place, a half step
-// has no order inside it, so every 4-node group of the grid is one thread's own work, and the fields
-// (24 B per node) and psi stay in the 126 MB L2 from step to step; a step then costs its L2 traffic
-// (72 B per node) and two barriers instead of three to six kernel launches.
+// has no order inside it, so every 4-node group of the grid is one thread's own work; a step costs its
+// traffic (72 B per node) and two barriers instead of three to six kernel launches. The fields (24 B per
+// node) and psi of up to about 4 M nodes stay in the 126 MB L2 from step to step, but that is not what
+// bounds it: 121^3 takes 15.1 ps a node, 201^3 15.6, 261^3 14.9, where the march takes 10.7 at 513^3. A
+// half step's chain does: class ids, L2 loads, the arithmetic, the barrier.
 //
 // Phase A of step n: new H from E (psi of H included); the records that read E after step n - 1
 // (port voltages, running DFTs of E, the NTFF box's M); each design edge's E^n.
