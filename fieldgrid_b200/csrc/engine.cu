@@ -2495,7 +2495,8 @@ int wait_error(int flag, std::string& err) {
 int session_check(Session* s, std::string& err) {
     if (!s->unchecked) return FG_OK;
     int flag = 0;
-    FG_CUDA(cudaMemcpy(&flag, s->error, sizeof(int), cudaMemcpyDeviceToHost));
+    FG_CUDA(cudaMemcpyAsync(&flag, s->error, sizeof(int), cudaMemcpyDeviceToHost, s->stream));   // no other stream is waited for
+    FG_CUDA(cudaStreamSynchronize(s->stream));
     if (flag) return wait_error(flag, err);
     s->unchecked = false;
     return FG_OK;
