@@ -1898,12 +1898,18 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     need += carve_size(cp.own.size() * sizeof(int2));
     // the device's spare arena serves when it holds the need with at most a quarter (+64 MB) more
     Gpu* gp = s->gpu;
-    if (gp->spare && !(gp->spare_bytes >= need && gp->spare_bytes <= need + need / 4 + (size_t(64) << 20))) {
-        cudaFree(gp->spare);
+    void* spare = nullptr;
+    {
+        std::lock_guard<std::mutex> hold(gp->spare_lock);
+        if (gp->spare && gp->spare_bytes >= need && gp->spare_bytes <= need + need / 4 + (size_t(64) << 20)) spare = gp->spare;
+        else if (gp->spare) cudaFree(gp->spare);
         gp->spare = nullptr;
         gp->spare_bytes = 0;
     }
-    if (!gp->spare) {
+    if (spare) {
+        s->arena = static_cast<char*>(spare);
+        s->arena_bytes = need;
+    } else {
         size_t free_b = 0, total_b = 0;
         FG_CUDA(cudaMemGetInfo(&free_b, &total_b));
         if (need + (size_t(256) << 20) > free_b) {
@@ -1916,13 +1922,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
         }
     }
     FG_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
-    if (gp->spare) {
-        s->arena = static_cast<char*>(gp->spare);
-        gp->spare = nullptr;
-        gp->spare_bytes = 0;
-    } else {
-        FG_CUDA(cudaMalloc(&s->arena, need));
-    }
+    if (!spare) FG_CUDA(cudaMalloc(&s->arena, need));
     clk.mark("malloc");
     s->arena_bytes = need;
     char* cur = s->arena;
@@ -2375,10 +2375,12 @@ void session_free(Session* s) {
     }
     if (s->arena) {   // kept as the device's spare (the stream is idle), or released
         Gpu* gp = s->gpu;
-        if (gp && !gp->spare) {
+        std::unique_lock<std::mutex> hold(gp->spare_lock);
+        if (!gp->spare) {
             gp->spare = s->arena;
             gp->spare_bytes = s->arena_bytes;
         } else {
+            hold.unlock();
             cudaFree(s->arena);
         }
     }

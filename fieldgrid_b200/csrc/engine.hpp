@@ -51,6 +51,7 @@ struct Gpu {
     // size (runs of one grid after another skip the allocation and its release)
     void* spare = nullptr;
     size_t spare_bytes = 0;
+    std::mutex spare_lock;                    // its taking and giving back
 };
 
 // Copies `bytes` from pageable host memory to the device through the Gpu's pinned staging buffers

@@ -414,6 +414,7 @@ class Session:
         _check(L.fg_session_new(None if g is None else g._h, sim._h, driven, C.byref(self._pl),
                                 C.byref(self._xs.struct), C.byref(out), err, ERRLEN), err)
         self._h = out
+        self._gpu = g             # the device handle outlives the session
         self.dims = sim.dims()
 
     def step(self, k: int) -> None:
@@ -724,6 +725,7 @@ class Batch:
         code = lib().fg_batch_new(g._h, hs, dv, pl, n, max_steps, C.byref(opt), C.byref(out), err, ERRLEN)
         _check(code, err)
         self._h = out
+        self._gpu = g             # the device handle outlives the batch
         self.size = n
 
     def step(self, k: int) -> None:
