@@ -84,7 +84,7 @@ constexpr int SHELL_THREADS = 256;   // 8 rows per block
 // Both are held to 64 registers (4 blocks per SM, 32 warps: a few bytes spill) for more loads in flight.
 // k_shell_h: 10 % faster at 512^3 than at its natural 80 registers (3 blocks). k_shell_e: 196 us at 80
 // registers with psi loaded for the live edges only, two dependent loads (class id, class) behind the
-// rest; 180 with psi loaded at once, 171 at 64 registers on top (583 MB, 3.4 TB/s; the merged batch launch, 112
+// rest; 180 with psi loaded at once, 171 at 64 registers on top (622 MB, 3.8 TB/s; the merged batch launch, 112
 // registers before: 851 -> 800 us a step of 12 grids); class ids a row's
 // pass ahead cost registers (254 at 2 blocks per SM, 174 at 3, 181 at 4).
 
