@@ -134,6 +134,7 @@ struct FluxJob {
     std::vector<int4> edges;
     uint64_t N = 0, L = 0, S = 0;
     bool ckpt = false, sep = false;
+    bool debye_groups = true; // RunSpec's
     bool resident = false;    // the sweep as resident launches (adjoint_resident.cuh)
     int* dwin = nullptr;      // of its Debye edges on the flux plane
     uint8_t* wmask = nullptr;
@@ -157,7 +158,10 @@ struct FluxJob {
         return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - a).count();
     }
 
-    ~FluxJob() {
+    ~FluxJob() { release(); }
+
+    // gives everything on the device back, so that prepare can start again
+    void release() {
         if (gpu) cudaSetDevice(gpu->device);
         if (sw) cudaStreamSynchronize(sw);
         if (s) cudaStreamSynchronize(s->stream);
@@ -170,6 +174,17 @@ struct FluxJob {
         cudaFree(gb);
         cudaFree(ck_mem);
         session_free(s);
+        evs.clear();
+        cks.clear();
+        edges.clear();
+        info.clear();
+        sw = nullptr;
+        s = nullptr;
+        for (auto** p : {&lE[0], &lE[1], &lH[0], &lH[1], &lpsi[0], &lpsi[1], &dw, &cam, &cbm, &lds, &lold}) *p = nullptr;
+        dwin = nullptr;
+        wmask = nullptr;
+        ga = gb = nullptr;
+        ck_mem = nullptr;
     }
 
     int event(cudaEvent_t* e, bool timing) {
@@ -195,10 +210,21 @@ struct FluxJob {
         return uint64_t(N) * info.size() * 8 <= per * S + 2 * L * info.size() * 8;
     }
 
-    // checks, the session, the checkpoints and the adjoint buffers
-    int prepare() {
+    bool out_of_memory(int rc) const {
+        return rc == FG_ERR_TOO_LARGE || (rc == FG_ERR_CUDA && err.find("out of memory") != std::string::npos);
+    }
+
+    // checks, the session, the checkpoints and the adjoint buffers. `alone`: no other job's memory will be
+    // given back, so a grid with Debye media that does not fit is tried without the resident steps' layout
+    int prepare(bool alone) {
         const auto p0 = std::chrono::steady_clock::now();
-        const int rc = prepare_();
+        int rc = prepare_();
+        if (rc && alone && out_of_memory(rc) && !sim->debye_edges.empty()) {
+            release();
+            cudaGetLastError();
+            debye_groups = false;
+            rc = prepare_();
+        }
         res.setup_ms = ms_since(p0);
         return rc;
     }
@@ -239,6 +265,7 @@ struct FluxJob {
         rs.has_plane_k = true;
         rs.plane_k = sp.plane_k;
         rs.fused = true;
+        rs.debye_groups = debye_groups;
         for (const auto& e : info) edges.push_back(e.at);
         rs.design = want_grad ? &edges : nullptr;
         rs.hist_cap = want_grad ? int(std::min<uint64_t>(S > 1 ? 2 * L : L, N)) : 0;   // checkpoints: a ring of two segments
@@ -628,7 +655,7 @@ int flux_gradient(Gpu* gpu, const HostSim& sim, uint64_t driven, double f0, doub
     j.fc = fc;
     j.sp = sp;
     j.want_grad = want_grad;
-    int rc = j.prepare();
+    int rc = j.prepare(true);
     if (!rc) rc = j.forward();
     if (!rc) rc = j.objective();
     if (!rc && want_grad) rc = j.backward();
@@ -684,12 +711,10 @@ int flux_gradient_batch(Gpu* gpu, const std::vector<const HostSim*>& sims, const
             j->fc = pulses[q].second;
             j->sp = specs[q];
             j->want_grad = true;
-            if ((rc = j->prepare())) {
+            if ((rc = j->prepare(G.empty() && !holding))) {
                 // out of device memory beside jobs already in flight: this job waits for a later
                 // group (its partial buffers go with it); alone, the error stands
-                const bool oom = rc == FG_ERR_TOO_LARGE ||
-                                 (rc == FG_ERR_CUDA && j->err.find("out of memory") != std::string::npos);
-                if (oom && (!G.empty() || holding)) {
+                if (j->out_of_memory(rc) && (!G.empty() || holding)) {
                     j.reset();
                     cudaGetLastError();
                     rc = FG_OK;

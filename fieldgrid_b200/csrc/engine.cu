@@ -1614,7 +1614,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     if (!gpu) { err = "no GPU: this engine has no CPU path"; return FG_ERR_NO_DEVICE; }
     FG_CUDA(cudaSetDevice(gpu->device));
     if (rs.driven >= sim.port_src.size()) { err = "the driven port does not exist"; return FG_ERR_INVALID; }
-    auto s = std::make_unique<Session>();
+    std::unique_ptr<Session, void (*)(Session*)> s(new Session, session_free);   // what it holds goes with a failure
     s->gpu = gpu;
     s->fused = rs.fused;
     const size_t n0 = sim.n[0], n1 = sim.n[1], n2 = sim.n[2], nn = sim.nn;

@@ -76,3 +76,40 @@ def test_a_grid_is_not_refused_for_the_resident_layout(gpu, monkeypatch):
         del hog
         torch.cuda.empty_cache()
         session(small).close()
+
+
+def test_a_gradient_is_not_refused_for_the_resident_layout(gpu, monkeypatch):
+    """The session fits with the layout, the sweep's buffers behind it only without."""
+    import torch
+
+    n = CELLS
+    one = np.ones(n ** 3, np.float32)
+    deb, design = one.copy().reshape(n, n, n), (slice(72, 78),) * 2 + (slice(40, 44),)
+    deb[68:82, 68:82, 36:48] = 0.0   # no Debye edge reaches the design
+    poles = fdtd.Debye([(1e9 * 2.0 ** q, 1.0 / POLES) for q in range(POLES)])
+    grid = Grid.uniform((0.0,) * 3, (n * 1e-3,) * 3, (n,) * 3, 8)
+    ports = [fdtd.PortDef("a", [[fdtd.Edge(2, (75, 75, 30))]], 50.0)]
+    sim = fdtd.Sim.try_new(grid, fdtd.Materials(2 + deb, 0 * one, 1 + deb, deb), None, [], ports, [],
+                           fdtd.Media(fdtd.Sheets(), poles, []))
+    pulse = fdtd.Pulse(10e9, 5e9)
+    spec = fdtd.FluxSpec(tuple(d.start for d in design), tuple(d.stop for d in design), 50, 10e9, 40)
+    want = fdtd.flux_gradient(gpu, sim, 0, pulse, spec)
+    sizes = []
+    for route in ("1", "0"):
+        monkeypatch.setenv("FIELDGRID_RESIDENT", route)
+        s = fdtd.Session(gpu, sim, 0, pulse, fdtd.Extras(max_steps=40, freqs=[10e9], plane_k=50, fused_e=True))
+        sizes.append(s.device_bytes)
+        s.close()
+    monkeypatch.delenv("FIELDGRID_RESIDENT")
+    small = _sim(20, 1)
+    fdtd.Session(gpu, small, 0, pulse, fdtd.Extras(max_steps=4, fused_e=True)).close()
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (sizes[0] + (300 << 20)), dtype=torch.uint8, device="cuda")
+    try:
+        for _ in range(2):   # the second finds what the first gave back
+            got = fdtd.flux_gradient(gpu, sim, 0, pulse, spec)
+            assert got.objective == want.objective and np.abs(want.grad_eps).max() > 0
+            assert np.array_equal(got.grad_eps, want.grad_eps) and np.array_equal(got.grad_sigma, want.grad_sigma)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
