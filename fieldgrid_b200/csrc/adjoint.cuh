@@ -615,7 +615,6 @@ struct FluxJob {
         FG_CUDA(cudaStreamSynchronize(sw));
         FG_CUDA(cudaStreamSynchronize(s->stream));
         res.backward_ms = ms_since(b0);
-        s->unchecked = true;   // the re-runs and the sweep
         if (const int rc = session_check(s, err)) return rc;
         for (auto& pr : t_rec) { float x = 0; FG_CUDA(cudaEventElapsedTime(&x, pr.first, pr.second)); res.recompute_ms += x; }
         for (auto& pr : t_sw) { float x = 0; FG_CUDA(cudaEventElapsedTime(&x, pr.first, pr.second)); res.adjoint_ms += x; }

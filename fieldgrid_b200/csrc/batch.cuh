@@ -177,31 +177,13 @@ struct Batch {
     // resident mode: the launches that share the SMs (0: off); the graphs keep `shape` for short calls
     int share = 0;
     bool resident_ok = false;
-    int** d_errors = nullptr;          // the grids' error words, and behind them their union
-    bool unchecked = false;            // steps enqueued since they were last read
 };
 
-__global__ void k_batch_errors(int* const* __restrict__ words, int n, int* __restrict__ out) {
-    int flag = 0;
-    for (int q = threadIdx.x; q < n; q += blockDim.x) flag |= *words[q];
-    flag = __reduce_or_sync(0xffffffffu, flag);
-    if (threadIdx.x == 0) *out = flag;
-}
-
-// The grids' error words once the steps enqueued so far have finished (session_check for the whole batch).
+// Waits for the steps enqueued so far and looks at every grid's error word.
 int batch_check(Batch& B, std::string& err) {
-    if (!B.unchecked) {
-        FG_CUDA(cudaStreamSynchronize(B.stream));
-        return FG_OK;
-    }
-    const int n = int(B.s.size());
-    int flag = 0;
-    k_batch_errors<<<1, 32, 0, B.stream>>>(B.d_errors, n, reinterpret_cast<int*>(B.d_errors + n));
-    FG_CUDA(cudaGetLastError());
-    FG_CUDA(cudaMemcpyAsync(&flag, B.d_errors + n, sizeof(int), cudaMemcpyDeviceToHost, B.stream));
     FG_CUDA(cudaStreamSynchronize(B.stream));
-    if (flag) return wait_error(flag, err);
-    B.unchecked = false;
+    for (const Session* s : B.s)
+        if (const int rc = session_check(s, err)) return rc;
     return FG_OK;
 }
 
@@ -496,7 +478,6 @@ void batch_free(Batch* B) {
     cudaFree(B->d_edges);
     cudaFree(B->d_ports);
     cudaFree(B->d_queue);
-    cudaFree(B->d_errors);
     cudaFree(B->d_tma);
     cudaFree(B->d_tma_block);
     cudaFree(B->d_shell);
@@ -547,7 +528,6 @@ int batch_reset(Batch& B, std::string& err) {
 
 int batch_step(Batch& B, uint64_t k, std::string& err) {
     FG_CUDA(cudaSetDevice(B.gpu->device));
-    B.unchecked = true;
     uint64_t done = 0;
     while (done < k) {
         const int parity = int(B.steps & 1);
@@ -653,15 +633,11 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
     FG_CUDA(cudaMalloc(&B->d_edges, (n + 1) * 8));
     FG_CUDA(cudaMalloc(&B->d_ports, (n + 1) * 8));
     FG_CUDA(cudaMalloc(&B->d_queue, 8));
-    FG_CUDA(cudaMalloc(&B->d_errors, (n + 1) * 8));
     FG_CUDA(cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming));
     B->join.assign(n, nullptr);
     for (auto& e : B->join) FG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     FG_CUDA(cudaMemcpy(B->d_edges, edges.data(), (n + 1) * 8, cudaMemcpyHostToDevice));
     FG_CUDA(cudaMemcpy(B->d_ports, ports.data(), (n + 1) * 8, cudaMemcpyHostToDevice));
-    std::vector<int*> words;
-    for (const Session* s : B->s) words.push_back(s->error);
-    FG_CUDA(cudaMemcpy(B->d_errors, words.data(), n * 8, cudaMemcpyHostToDevice));
     int rc = batch_merged_setup(*B, err);
     if (rc) return rc;
     // the tuner: each candidate runs a warm-up step then a timed block of steps from the live state
@@ -708,7 +684,7 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
                 FG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
             }
             cudaGraphExecDestroy(gx);
-            B->unchecked = true;   // a wait that ran out ends a trial early: no time of that is compared
+            // a wait that ran out ends a trial early: no time of that is compared
             if ((rc = batch_check(*B, err))) break;
             B->trials.push_back({sh, ms / timed});
             if (ms / timed < best_ms) { best_ms = ms / timed; best = sh; }
@@ -726,7 +702,6 @@ int batch_new(Gpu* gpu, const std::vector<const HostSim*>& sims, const std::vect
                 FG_CUDA(cudaEventSynchronize(e1));
             }
             float ms = 0;
-            B->unchecked = true;
             if (rc || (rc = batch_check(*B, err))) break;
             FG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
             B->trials.push_back({BatchShape{BATCH_RESIDENT, sh, 0}, ms / float(many)});

@@ -77,7 +77,25 @@ void gpu_close(Gpu* g) {
         }
         if (g->stage[b]) cudaFreeHost(g->stage[b]);
     }
+    for (int* p : g->word_pages) cudaFreeHost(p);
     delete g;
+}
+
+// A cleared error word for a session, and its address on the device.
+static int take_word(Gpu* g, int** host, int** device, std::string& err) {
+    std::lock_guard<std::mutex> hold(g->word_lock);
+    if (g->words.empty()) {
+        constexpr int PAGE = 1024;
+        int* p = nullptr;
+        FG_CUDA(cudaHostAlloc(&p, PAGE * sizeof(int), cudaHostAllocMapped));
+        g->word_pages.push_back(p);
+        for (int q = PAGE; q-- > 0;) g->words.push_back(p + q);
+    }
+    FG_CUDA(cudaHostGetDevicePointer(device, g->words.back(), 0));
+    *host = g->words.back();
+    g->words.pop_back();
+    **host = 0;
+    return FG_OK;
 }
 
 static constexpr size_t STAGE_BYTES = size_t(32) << 20;
@@ -240,7 +258,7 @@ struct Session {
     float* debye_state = nullptr;
     float* debye_table = nullptr;
     double* partial = nullptr;
-    int* error = nullptr;           // set by a kernel whose bounded wait ran out
+    int *error = nullptr, *error_word = nullptr;   // set by a kernel whose bounded wait ran out: on the device, on the host
     TmaPlan tma;                    // the TMA-fed fused step, when it applies
     uint8_t* local_ids = nullptr;   // per node: index into its block region's coefficient table
     int4* tma_blocks = nullptr;     // the TMA march's blocks over the clean box
@@ -304,7 +322,6 @@ struct Session {
     unsigned long long wait_ns = tma::WAIT_LIMIT_NS;
     int stall_plane = -1;
     bool stall_barrier = false;     // test knob of the resident kernels' grid barrier (ResArgs::late)
-    bool unchecked = false;         // steps enqueued since the error word was last read
     int2* tma_own = nullptr;        // per block of the one-step march: the rows it writes
     // ---- the two-step mode (stencil_tb2.cuh). Step t reads field set, z-slab psi slot and Debye
     // state slot t mod 3 and writes (t + 1) mod 3; the x/y slabs keep the one-step scheme (E in
@@ -1890,7 +1907,6 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     need += carve_size(std::max<size_t>(t_dft.size(), 1) * 4) * 2;
     need += carve_size(ENERGY_BLOCKS * 8);
     need += carve_size(64);
-    need += carve_size(64);
     const size_t local_tables = cp.blocks.size() * LOCAL_CLASSES * 6;
     if (s->local) need += carve_size(nnp) + carve_size(local_tables * 4);
     need += carve_size(64);
@@ -1921,6 +1937,7 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
             return FG_ERR_TOO_LARGE;
         }
     }
+    if (const int rw = take_word(gpu, &s->error_word, &s->error, err)) return rw;
     FG_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     if (!spare) FG_CUDA(cudaMalloc(&s->arena, need));
     clk.mark("malloc");
@@ -1974,7 +1991,6 @@ int session_new(Gpu* gpu, const HostSim& sim, const RunSpec& rs, Session** out, 
     sc.dft = d_dft;
     sc.far = d_far;
     s->partial = carve<double>(cur, ENERGY_BLOCKS);
-    s->error = carve<int>(cur, 16);
     s->res_bar = carve<unsigned>(cur, 16);
     if (s->local) {
         s->local_ids = carve<uint8_t>(cur, nnp);
@@ -2373,6 +2389,10 @@ void session_free(Session* s) {
         if (s->aux_ready[p]) cudaEventDestroy(s->aux_ready[p]);
         if (s->aux_done[p]) cudaEventDestroy(s->aux_done[p]);
     }
+    if (s->error_word) {
+        std::lock_guard<std::mutex> hold(s->gpu->word_lock);
+        s->gpu->words.push_back(s->error_word);
+    }
     if (s->arena) {   // kept as the device's spare (the stream is idle), or released
         Gpu* gp = s->gpu;
         std::unique_lock<std::mutex> hold(gp->spare_lock);
@@ -2433,7 +2453,6 @@ int session_reset(Session* s, std::string& err) {
 int session_step(Session* s, uint64_t k, std::string& err) {
     if (!s->slots && !s->resident && !s->graph_one[0]) { err = "this session steps only as part of a batch"; return FG_ERR_INVALID; }
     FG_CUDA(cudaSetDevice(s->gpu->device));
-    s->unchecked = true;
     uint64_t done = 0;
     if (s->resident) {
         while (done < k) {
@@ -2492,16 +2511,11 @@ int wait_error(int flag, std::string& err) {
     return FG_ERR_CUDA;
 }
 
-// The error word of the steps since the last look, once they have finished: the fields after a wait that
-// ran out are those of no step. The word stays set, so every later look reports it again.
-int session_check(Session* s, std::string& err) {
-    if (!s->unchecked) return FG_OK;
-    int flag = 0;
-    FG_CUDA(cudaMemcpyAsync(&flag, s->error, sizeof(int), cudaMemcpyDeviceToHost, s->stream));   // no other stream is waited for
-    FG_CUDA(cudaStreamSynchronize(s->stream));
-    if (flag) return wait_error(flag, err);
-    s->unchecked = false;
-    return FG_OK;
+// The error word of the steps that have finished (the caller has waited for them): the fields after a wait
+// that ran out are those of no step. The word stays set, so every later look reports it again.
+int session_check(const Session* s, std::string& err) {
+    const int flag = *static_cast<volatile int*>(s->error_word);
+    return flag ? wait_error(flag, err) : FG_OK;
 }
 
 int session_sync(Session* s, std::string& err) {
@@ -2634,7 +2648,6 @@ int session_kernel_times(Session* s, uint64_t steps, std::vector<std::pair<std::
     std::vector<int> counts;
     // the two-step mode times double steps (one stream) and reports each kernel's time per step
     const uint64_t per = s->slots ? 2 : 1;
-    s->unchecked = true;
     if (const int rc = debye_states(*s, false, s->stream, err)) return rc;
     for (uint64_t q = 0; q < steps; q += per) {
         marks.clear();

@@ -52,6 +52,10 @@ struct Gpu {
     void* spare = nullptr;
     size_t spare_bytes = 0;
     std::mutex spare_lock;                    // its taking and giving back
+    // error words of the device's sessions, in pinned pages that kernels write and the host reads without
+    // a copy: the pages, and the words no session has
+    std::vector<int*> word_pages, words;
+    std::mutex word_lock;
 };
 
 // Copies `bytes` from pageable host memory to the device through the Gpu's pinned staging buffers

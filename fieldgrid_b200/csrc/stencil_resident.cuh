@@ -202,7 +202,7 @@ __device__ __forceinline__ bool res_barrier(const ResArgs& a, unsigned target) {
                 asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
                 if (t0 == 0) t0 = t;
                 else if (t - t0 > a.wait_ns) {
-                    atomicExch(a.error, 3);
+                    *static_cast<volatile int*>(a.error) = 3;
                     bad = 1;
                     break;
                 }

@@ -280,7 +280,7 @@ __device__ __forceinline__ void tb2_march(const CUtensorMap& map_e, const CUtens
         for (int p = p_first; p <= p_last; ++p) {
             const int u = p - p_first, s = u % STAGES, n = u / STAGES;
             if (!tma::mbar_wait(&empty[s], uint32_t((n & 1) ^ 1), a.wait_ns)) {
-                atomicExch(a.error, 3);
+                *static_cast<volatile int*>(a.error) = 3;
                 // the copies already issued land before the block leaves (bounded waits)
                 for (int q = max(p_first, p - STAGES); q < p; ++q) {
                     const int uq = q - p_first;
@@ -432,7 +432,7 @@ __device__ __forceinline__ void tb2_march(const CUtensorMap& map_e, const CUtens
             }
         }
         if (tma::consumers_sync_or(bad, TB_CONSUMERS)) {
-            if (tid == 0) atomicExch(a.error, 4);
+            if (tid == 0) *static_cast<volatile int*>(a.error) = 4;
             return;
         }
 
@@ -523,7 +523,7 @@ __device__ __forceinline__ void tb2_march(const CUtensorMap& map_e, const CUtens
             }
         }
         if (tma::consumers_sync_or(bad, TB_CONSUMERS)) {
-            if (tid == 0) atomicExch(a.error, 4);
+            if (tid == 0) *static_cast<volatile int*>(a.error) = 4;
             return;
         }
 

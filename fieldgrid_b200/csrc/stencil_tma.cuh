@@ -481,7 +481,7 @@ __device__ __forceinline__ void tma_march(const CUtensorMap& map_e, const CUtens
         for (int p = p_first; p <= p_last; ++p) {
             const int u = p - p_first, s = u % STAGES, n = u / STAGES;
             if (!tma::mbar_wait(&empty[s], uint32_t((n & 1) ^ 1), a.wait_ns)) {
-                atomicExch(a.error, 1);
+                *static_cast<volatile int*>(a.error) = 1;
                 // the copies already issued land before the block leaves (bounded waits)
                 for (int q = max(p_first, p - STAGES); q < p; ++q) {
                     const int uq = q - p_first;
@@ -729,7 +729,7 @@ __device__ __forceinline__ void tma_march(const CUtensorMap& map_e, const CUtens
             }
         }
         if (tma::consumers_sync_or(bad, TMA_CONSUMERS)) {
-            if (tid == 0) atomicExch(a.error, 2);
+            if (tid == 0) *static_cast<volatile int*>(a.error) = 2;
             return;
         }
 
