@@ -130,7 +130,7 @@ int staged_fill(Gpu* g, void* dst, size_t bytes, cudaStream_t st, Fill&& fill) {
         if (e != cudaSuccess) return int(e);
         char* buf = static_cast<char*>(g->stage[b]);
         const long long parts = (long long)((n + (size_t(1) << 20) - 1) >> 20);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (parts > 1)
         for (long long q = 0; q < parts; ++q) {
             const size_t a = size_t(q) << 20, m = std::min(size_t(1) << 20, n - a);
             fill(buf + a, off + a, m);

@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -281,20 +282,22 @@ std::atomic<long long> far_kept{0};
 struct FarDevice {
     int device = 0;
     long long count = 0;
+    char* mem = nullptr;              // one allocation: the layout, and behind it the first call's work
     double *pos = nullptr, *jm = nullptr, *seqs = nullptr;
     FarGroup* groups = nullptr;
     bool lined = false;
     struct Run { int axis, len, seq, g0, g1; };   // groups of one sequence
     std::vector<Run> runs;
-    char* work = nullptr;             // the calls' directions, parts and partial sums, grown as needed
+    char *work = nullptr, *own_work = nullptr;   // the calls' directions, parts and partial sums; an allocation of its own once outgrown
     size_t work_bytes = 0;
-    long long bytes = 0, kept = 0;    // of the layout; what far_kept counts for this one
+    long long bytes = 0, kept = 0;    // allocated; what far_kept counts for this one
     ~FarDevice() {
         far_kept -= kept;
         int prev = 0;
         const bool back = cudaGetDevice(&prev) == cudaSuccess;
         cudaSetDevice(device);
-        for (void* p : {(void*)pos, (void*)jm, (void*)seqs, (void*)groups, (void*)work}) cudaFree(p);
+        cudaFree(mem);
+        if (own_work) cudaFree(own_work);
         if (back) cudaSetDevice(prev);
     }
 };
@@ -303,70 +306,74 @@ void far_device_free(FarDevice* d) { delete d; }
 
 namespace {
 
-int far_layout(Gpu* g, const double* pos, const double* area, const double* jm, uint64_t count, FarDevice& D, std::string& err) {
-    auto check = [&](cudaError_t e, const char* what) {
-        if (e != cudaSuccess) { err = std::string(what) + ": " + cudaGetErrorString(e); return false; }
-        return true;
-    };
-    D.device = g->device;
-    D.count = (long long)count;
+// The patches' lines in groups of four, where they form lines that share their sequences.
+void far_groups(const double* pos, uint64_t count, FarDevice& D, std::vector<FarGroup>& groups, std::vector<double>& seqs) {
     std::vector<Line> lines;
-    std::vector<double> seqs;
     D.lined = false;
     if (count > 0 && count < (uint64_t(1) << 31)) {
         find_lines(pos, int(count), lines, seqs);
         D.lined = lines.size() * 8 <= count;
     }
-    D.bytes = (long long)(13 * count * 8);
+    if (!D.lined) return;
+    // lines of one sequence, in their order, four to a group
+    std::stable_sort(lines.begin(), lines.end(), [](const Line& a, const Line& b) { return a.seq < b.seq; });
+    long long slots = 0;
+    for (size_t i = 0; i < lines.size();) {
+        size_t e = i;
+        while (e < lines.size() && lines[e].seq == lines[i].seq) ++e;
+        FarDevice::Run r{lines[i].axis, lines[i].len, lines[i].seq, int(groups.size()), 0};
+        for (size_t q = i; q < e; q += 4) {
+            FarGroup G{};
+            G.lines = int(std::min<size_t>(4, e - q));
+            for (int l = 0; l < 4; ++l) {
+                const Line& L = lines[q + size_t(l < G.lines ? l : 0)];
+                G.first[l] = L.first;
+                for (int x = 0; x < 3; ++x) G.base[l][x] = x == L.axis ? 0.0 : pos[3 * (size_t)L.first + x];
+            }
+            groups.push_back(G);
+        }
+        r.g1 = int(groups.size());
+        D.runs.push_back(r);
+        slots += (long long)((r.g1 - r.g0 + FAR_WARPS - 1) / FAR_WARPS) * FAR_WARPS * 4 * r.len;
+        i = e;
+    }
+    D.lined = D.runs.size() <= FAR_SEQUENCES && slots <= FAR_PADDING * (long long)count;
+}
+
+// Allocates and fills a handle's layout, with `work` bytes behind it.
+int far_layout(Gpu* g, const double* pos, const double* area, const double* jm, uint64_t count, FarDevice& D,
+               const std::vector<FarGroup>& groups, const std::vector<double>& seqs, size_t work, std::string& err) {
+    auto check = [&](cudaError_t e, const char* what) {
+        if (e != cudaSuccess) { err = std::string(what) + ": " + cudaGetErrorString(e); return false; }
+        return true;
+    };
+    auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+    const size_t jb = al(13 * count * 8), gb = D.lined ? al(groups.size() * sizeof(FarGroup)) : 0;
+    const size_t sb = D.lined ? al(seqs.size() * 8) : al(3 * count * 8);
+    if (!check(cudaMalloc(&D.mem, jb + gb + sb + work), "cudaMalloc")) return FG_ERR_CUDA;
+    D.bytes = (long long)(jb + gb + sb + work);
+    D.jm = reinterpret_cast<double*>(D.mem);
+    D.work = D.mem + jb + gb + sb;
+    D.work_bytes = work;
     // the currents, then their areas behind them for the products
-    if (!check(cudaMalloc(&D.jm, std::max<size_t>(13 * count, 1) * 8), "cudaMalloc")) return FG_ERR_CUDA;
     if (count) {
         double* a = D.jm + 12 * count;
         if (!check(cudaError_t(staged_upload(g, D.jm, jm, 12 * count * 8, nullptr)), "cudaMemcpy") ||
             !check(cudaError_t(staged_upload(g, a, area, count * 8, nullptr)), "cudaMemcpy"))
             return FG_ERR_CUDA;
-        k_far_areas<<<148 * 8, 256>>>(D.jm, a, (long long)count);
+        k_far_areas<<<unsigned(std::min<uint64_t>((12 * count + 255) / 256, 148 * 8)), 256>>>(D.jm, a, (long long)count);
         if (!check(cudaGetLastError(), "k_far_areas")) return FG_ERR_CUDA;
     }
-    std::vector<FarGroup> groups;
     if (D.lined) {
-        // lines of one sequence, in their order, four to a group
-        std::stable_sort(lines.begin(), lines.end(), [](const Line& a, const Line& b) { return a.seq < b.seq; });
-        long long slots = 0;
-        for (size_t i = 0; i < lines.size();) {
-            size_t e = i;
-            while (e < lines.size() && lines[e].seq == lines[i].seq) ++e;
-            FarDevice::Run r{lines[i].axis, lines[i].len, lines[i].seq, int(groups.size()), 0};
-            for (size_t q = i; q < e; q += 4) {
-                FarGroup G{};
-                G.lines = int(std::min<size_t>(4, e - q));
-                for (int l = 0; l < 4; ++l) {
-                    const Line& L = lines[q + size_t(l < G.lines ? l : 0)];
-                    G.first[l] = L.first;
-                    for (int x = 0; x < 3; ++x) G.base[l][x] = x == L.axis ? 0.0 : pos[3 * (size_t)L.first + x];
-                }
-                groups.push_back(G);
-            }
-            r.g1 = int(groups.size());
-            D.runs.push_back(r);
-            slots += (long long)((r.g1 - r.g0 + FAR_WARPS - 1) / FAR_WARPS) * FAR_WARPS * 4 * r.len;
-            i = e;
-        }
-        D.lined = D.runs.size() <= FAR_SEQUENCES && slots <= FAR_PADDING * (long long)count;
-    }
-    if (D.lined) {
-        D.bytes += (long long)(groups.size() * sizeof(FarGroup) + seqs.size() * 8);
-        if (!check(cudaMalloc(&D.groups, groups.size() * sizeof(FarGroup)), "cudaMalloc") ||
-            !check(cudaMalloc(&D.seqs, seqs.size() * 8), "cudaMalloc") ||
-            !check(cudaMemcpy(D.groups, groups.data(), groups.size() * sizeof(FarGroup), cudaMemcpyHostToDevice), "cudaMemcpy") ||
+        D.groups = reinterpret_cast<FarGroup*>(D.mem + jb);
+        D.seqs = reinterpret_cast<double*>(D.mem + jb + gb);
+        if (!check(cudaMemcpy(D.groups, groups.data(), groups.size() * sizeof(FarGroup), cudaMemcpyHostToDevice), "cudaMemcpy") ||
             !check(cudaMemcpy(D.seqs, seqs.data(), seqs.size() * 8, cudaMemcpyHostToDevice), "cudaMemcpy") ||
             !check(cudaFuncSetAttribute(k_far_lines, cudaFuncAttributeMaxDynamicSharedMemorySize, FAR_SMEM), "cudaFuncSetAttribute"))
             return FG_ERR_CUDA;
-    } else {
-        D.bytes += (long long)(3 * count * 8);
-        if (!check(cudaMalloc(&D.pos, std::max<size_t>(3 * count, 1) * 8), "cudaMalloc") ||
-            !check(cudaMemcpy(D.pos, pos, 3 * count * 8, cudaMemcpyHostToDevice), "cudaMemcpy"))
-            return FG_ERR_CUDA;
+    } else if (count) {
+        D.pos = reinterpret_cast<double*>(D.mem + jb);
+        if (!check(cudaMemcpy(D.pos, pos, 3 * count * 8, cudaMemcpyHostToDevice), "cudaMemcpy")) return FG_ERR_CUDA;
     }
     return FG_OK;
 }
@@ -381,17 +388,19 @@ int far_field_gpu(Gpu* g, std::vector<FarDevice*>& devices, const double* pos, c
         return true;
     };
     if (!check(cudaSetDevice(g->device), "cudaSetDevice")) return FG_ERR_CUDA;
-    FarDevice** dev = nullptr;   // the handle's layout on this device, made on first use
-    for (auto& d : devices)
-        if (d->device == g->device) dev = &d;
+    FarDevice* dev = nullptr;   // the handle's layout on this device, made on first use
+    for (FarDevice* d : devices)
+        if (d->device == g->device) dev = d;
+    std::unique_ptr<FarDevice> made;
+    std::vector<FarGroup> groups;
+    std::vector<double> seqs;
     if (!dev) {
-        auto* D = new FarDevice;
-        const int rc = far_layout(g, pos, area, jm, count, *D, err);
-        if (rc) { delete D; return rc; }
-        devices.push_back(D);
-        dev = &devices.back();
+        made.reset(dev = new FarDevice);
+        dev->device = g->device;
+        dev->count = (long long)count;
+        far_groups(pos, count, *dev, groups, seqs);
     }
-    FarDevice& D = **dev;
+    FarDevice& D = *dev;
     const double kw = 2.0 * 3.14159265358979323846 * freq / 299792458.0;
     constexpr uint64_t MOST = 65535;   // directions at a time
     const int m0 = int(std::min<uint64_t>(n, MOST));
@@ -400,13 +409,13 @@ int far_field_gpu(Gpu* g, std::vector<FarDevice*>& devices, const double* pos, c
     // less work than one pass per SM, a group a block
     std::vector<FarPart> parts;
     if (D.lined) {
-        long long work = 0, groups = 0;
+        long long work = 0, all = 0;
         for (const auto& r : D.runs) {
             work += (long long)(r.g1 - r.g0) * r.len;
-            groups += r.g1 - r.g0;
+            all += r.g1 - r.g0;
         }
         const long long tiles = (m0 + 31) / 32, per = std::max<long long>(work * tiles / (148 * 7), 1);
-        const bool few = tiles * groups < 148 * FAR_WARPS;
+        const bool few = tiles * all < 148 * FAR_WARPS;
         for (const auto& r : D.runs) {
             const long long pass = (long long)r.len * FAR_WARPS;
             const int m = few ? 1 : FAR_WARPS * int(std::max<long long>(1, (per + pass / 2) / pass));
@@ -418,12 +427,20 @@ int far_field_gpu(Gpu* g, std::vector<FarDevice*>& devices, const double* pos, c
     const int ms = int(std::min<uint64_t>(n, step));
     const size_t pb = (parts.size() * sizeof(FarPart) + 255) & ~size_t(255);
     const size_t bytes = pb + (size_t(9) + size_t(12) * parts.size()) * size_t(ms) * 8 + 256;
-    if (D.work_bytes < bytes) {
-        cudaFree(D.work);
-        D.work = nullptr;
+    if (made) {
+        if (const int rc = far_layout(g, pos, area, jm, count, D, groups, seqs, bytes, err)) return rc;
+        devices.push_back(made.release());
+    } else if (D.work_bytes < bytes) {
+        if (D.own_work) {
+            cudaFree(D.own_work);
+            D.bytes -= (long long)D.work_bytes;
+        }
+        D.work = D.own_work = nullptr;
         D.work_bytes = 0;
-        if (!check(cudaMalloc(&D.work, bytes), "cudaMalloc")) return FG_ERR_CUDA;
+        if (!check(cudaMalloc(&D.own_work, bytes), "cudaMalloc")) return FG_ERR_CUDA;
+        D.work = D.own_work;
         D.work_bytes = bytes;
+        D.bytes += (long long)bytes;
     }
     char* buf = D.work;
     double* d_dirs = reinterpret_cast<double*>(buf + pb);
@@ -446,11 +463,11 @@ int far_field_gpu(Gpu* g, std::vector<FarDevice*>& devices, const double* pos, c
              check(cudaMemcpyAsync(out + 6 * first, d_out, size_t(m) * 48, cudaMemcpyDeviceToHost, nullptr), "cudaMemcpy");
     }
     ok = check(cudaStreamSynchronize(nullptr), "far field") && ok;
-    const long long now = D.bytes + (long long)D.work_bytes, all = far_kept += now - D.kept;
-    D.kept = now;
+    const long long all = far_kept += D.bytes - D.kept;
+    D.kept = D.bytes;
     if (all > FAR_KEEP) {
-        devices.erase(std::find(devices.begin(), devices.end(), &D));
-        delete &D;
+        devices.erase(std::find(devices.begin(), devices.end(), dev));
+        delete dev;
     }
     return ok ? FG_OK : FG_ERR_CUDA;
 }
