@@ -47,7 +47,7 @@ struct FastDiv {
         while ((1ull << s) < div) ++s;
         m = ((1ull << (32 + s)) + div - 1) / div;
     }
-    __device__ __forceinline__ unsigned operator()(unsigned n) const {
+    __host__ __device__ __forceinline__ unsigned operator()(unsigned n) const {
         return unsigned(((unsigned long long)n * m) >> (32 + s));
     }
 };
