@@ -11,7 +11,7 @@
 // four lines at a time (a table entry serves four, the lines' currents come as broadcasts, staged with
 // cp.async), and a block's warps share the table of 32 directions. Its floor is the FP64 rate: 174,760
 // patches x 2664 directions are 11.2 G multiply-adds, 0.6 ms at 64 per SM and clock; a repeated call takes
-// 2.0 ms, the first on a handle, which lays its patches out on the device, 5 to 6; a block per direction took
+// 2.0 ms, the first on a handle, which lays its patches out on the device, 4.5 to 6; a block per direction took
 // 13.4 with its copies each time.
 // Patches that do not come in lines (fewer than 8 per line on average), or whose lines hardly share their
 // sequences (FAR_SEQUENCES, FAR_PADDING), go through k_far_field, a block per direction, which forms every
